@@ -23,7 +23,8 @@
  *   dlrb200_workspace_bytes- the per-call torch allocations of those entry
  *                            points (cooperative.cu:608-614), hoisted to the
  *                            caller.
- *   dlrb200_query          - the per-batch tile tables of the Python wrappers
+ *   dlrb200_query, dlrb200_query_call
+ *                          - the per-batch tile tables of the Python wrappers
  *                            (kernels/kernels/cooperative.py:24-38) and
  *                            kernels/registry.py:130-135.
  *   dlrb200_fold_weights   - pack_dlrnet_weights (kernels/reference.py:68-91).
@@ -66,6 +67,7 @@ extern "C" {
 #define DLRB200_PATH_CLUSTER_SMALL 3 /* small batch: one cluster per 2 rows, exchange in distributed shared memory */
 #define DLRB200_PATH_STREAMED 4 /* large batch: one CTA per 128-row tile, activations streamed through shared memory */
 #define DLRB200_PATH_STRIPED_CLUSTERS 6 /* small batch: width-striped CTAs in clusters of 8, exchange first inside the cluster, then through L2 */
+#define DLRB200_PATH_RESIDENT 7 /* small batch: clusters of d/256 (or d/320) CTAs keep their rows in registers, exchange in distributed shared memory */
 #define DLRB200_PATH_STREAMED_PAIRS 5 /* large batch: one CTA pair per 256-row tile (tcgen05 cta_group::2), activations streamed */
 
 typedef struct dlrb200_plan {
@@ -73,8 +75,8 @@ typedef struct dlrb200_plan {
     int grid;           /* CTAs per launch */
     int cluster;        /* CTAs per cluster (1 = none) */
     int stripe_cols;    /* columns of the model width owned by one CTA */
-    int rows_per_pass;  /* token rows handled by one launch (striped) or one cluster tile */
-    int passes;         /* striped path: launches per forward; cluster and streamed paths: waves of row tiles in the one launch */
+    int rows_per_pass;  /* token rows handled by one launch (striped) or one cluster */
+    int passes;         /* striped path: launches per forward; other paths: waves of row tiles in the one launch */
     int stages;         /* depth of the weight ring, in layers (striped) or tiles (cluster) */
     size_t smem_bytes;  /* dynamic shared memory per CTA */
     size_t workspace_bytes;
@@ -96,9 +98,15 @@ DLRB200_API int dlrb200_last_cuda_error(void);
  * must not overlap on the GPU.  Returns 0 for an unsupported shape. */
 DLRB200_API size_t dlrb200_workspace_bytes(int M, int d, int r, int L);
 
-/* How a forward of this shape would run on the current device.  Launches
- * nothing.  Returns DLRB200_ERR_UNSUPPORTED_SHAPE / _OCCUPANCY when it cannot. */
+/* How the kernels that take any shape (paths 1 to 6) would run a forward of
+ * this shape on the current device.  Launches nothing.  Returns
+ * DLRB200_ERR_UNSUPPORTED_SHAPE / _OCCUPANCY when they cannot. */
 DLRB200_API int dlrb200_query(int M, int d, int r, int L, dlrb200_plan* plan);
+
+/* What dlrb200_forward launches for a call of this shape: the plan of
+ * dlrb200_query, or that of the resident-cluster kernel (path 7), which takes
+ * small and medium batches of the shapes it is built for. */
+DLRB200_API int dlrb200_query_call(int M, int d, int r, int L, dlrb200_plan* plan);
 
 /* y = DLRNet(x).
  *   x, y        (M, d) bf16 row-major device buffers, 16-byte aligned; may not alias.

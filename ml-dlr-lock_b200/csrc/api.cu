@@ -8,6 +8,7 @@
 #include "decode.h"
 #include "decode_cluster.h"
 #include "decode_tl.h"
+#include "resident.h"
 #include "stream.h"
 #include "stream_pair.h"
 
@@ -254,6 +255,7 @@ int check_shape(int M, int d, int r, int L) {
 // Shapes the cluster kernel does not cover (d > 4096, d not a multiple of 512, r > d / 32) stream.
 struct RouteEntry {
     int tiles, d, r, L, sms, path;         // the plans depend on M only through the number of 128-row tiles
+    double us;                             // estimated time of that path
 };
 constexpr int kRouteSlots = 32;
 RouteEntry g_route[kRouteSlots];
@@ -263,7 +265,8 @@ std::mutex g_route_mutex;
 
 // DLRB200_PATH_* of the kernel that serves M > 64 rows, or 0 when none of the large-batch kernels applies
 // (then the striped kernel runs in 64-row launches).
-int large_batch_path(int M, int d, int r, int L, const DevInfo& di) {
+int large_batch_path(int M, int d, int r, int L, const DevInfo& di, double* estimate_us = nullptr) {
+    if (estimate_us) *estimate_us = 1e30;
     const int forced = env_int("DLRB200_FORCE_PATH", 0);
     if (M <= 64) return 0;
     const bool can_stream = dlr::stream_supported(d, r);
@@ -273,13 +276,16 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di) {
     if (forced == DLRB200_PATH_STREAMED_PAIRS) return can_pair ? forced : 0;
     if (forced == DLRB200_PATH_CLUSTER) return can_cluster ? forced : 0;
     if (forced != 0) return 0;
-    if (!can_stream && !can_pair) return can_cluster ? DLRB200_PATH_CLUSTER : 0;
+    if (!can_stream && !can_pair && !can_cluster) return 0;
     const int tiles = (M + 127) / 128;
     {   // the plans below ask the driver for occupancy: remember the answer per shape
         std::lock_guard<std::mutex> lock(g_route_mutex);
         for (int i = 0; i < g_route_n; ++i) {
             const RouteEntry& e = g_route[i];
-            if (e.tiles == tiles && e.d == d && e.r == r && e.L == L && e.sms == di.num_sms) return e.path;
+            if (e.tiles == tiles && e.d == d && e.r == r && e.L == L && e.sms == di.num_sms) {
+                if (estimate_us) *estimate_us = e.us;
+                return e.path;
+            }
         }
     }
     double best = 1e30;
@@ -288,7 +294,7 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di) {
     if (can_cluster) {
         std::memset(&pl, 0, sizeof(pl));
         if (dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, &pl) == DLRB200_OK) {
-            best = 0.97 * double(pl.passes) * L * (r >= 128 ? 8.2 : 6.4);     // ties go to the cluster kernel
+            best = 0.97 * double(pl.passes) * L * (r >= 128 ? 8.2 : (r >= 64 ? 6.4 : 5.5));     // ties go to the cluster kernel
             path = DLRB200_PATH_CLUSTER;
         }
     }
@@ -296,7 +302,7 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di) {
         std::memset(&pl, 0, sizeof(pl));
         if (dlr::stream_plan(M, d, r, L, di.num_sms, di.smem_optin, &pl) == DLRB200_OK) {
             const double t_pass = pl.cluster >= 4 ? 6.8 : (pl.cluster == 2 ? 5.5 : 2.5);
-            double t = double(pl.passes) * (L + 1) * (double(d / 128 / pl.cluster) * (r >= 128 ? 1.26 : 1.15) + t_pass);
+            double t = double(pl.passes) * (L + 1) * (double(d / 128 / pl.cluster) * (r >= 256 ? 3.05 : (r >= 128 ? 1.26 : 1.15)) + t_pass);
             if (pl.cluster == 1 && pl.grid > 100 && 4.0 * L * d * r > 100e6) t *= 1.3;
             // every layer rewrites the rows in flight in place: once they outgrow L2 (beside the weight stream)
             // each layer's traffic goes to DRAM (measured at d = 4096: 12288 / 16384 / 18944 rows in flight
@@ -321,10 +327,29 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di) {
         }
     }
     std::lock_guard<std::mutex> lock(g_route_mutex);
-    g_route[g_route_next] = RouteEntry{tiles, d, r, L, di.num_sms, path};
+    g_route[g_route_next] = RouteEntry{tiles, d, r, L, di.num_sms, path, best};
+    if (estimate_us) *estimate_us = best;
     g_route_next = (g_route_next + 1) % kRouteSlots;
     if (g_route_n < kRouteSlots) ++g_route_n;
     return path;
+}
+
+// Calls that the resident-cluster kernel serves instead of the kernel planned above, where it covers the shape: batches of
+// up to 64 rows (measured against the best of the others, us: d = 1024 110 / 281 at one row, 112 / 295 at 64; d = 2048
+// 151 / 332 at 8, 162 / 767 at 64; d = 4096 224 / 323 at one row, 237 / 524 at 16, 360 / 1093 at 64; at d = 5120 each of its
+// 16 CTAs pulls 328 KB a layer and the striped kernel's 80 are faster up to a dozen rows: 674 / 445 at one row, 648 / 828 at
+// 12), and beyond that wherever waves of small row groups end before the large-batch kernel's one pass over a tile: both
+// sides estimated from measured times.
+bool use_resident(int M, int d, int r, int L, const DevInfo& di, dlrb200_plan* plan = nullptr) {
+    const int forced = env_int("DLRB200_FORCE_PATH", 0);
+    if (!dlr::resident_supported(d, r) || (forced != 0 && forced != DLRB200_PATH_RESIDENT)) return false;
+    if (forced == 0 && M <= 64 && r >= 256 && M < 12) return false;
+    const double us = dlr::resident_estimate_us(M, d, r, L, di.smem_optin, plan);
+    if (us >= 1e30) return false;
+    if (forced != 0 || M <= 64) return true;
+    double other = 1e30;
+    large_batch_path(M, d, r, L, di, &other);
+    return us < 0.75 * other;             // (near a tie the large-batch kernel, whose time does not grow with the rows)
 }
 
 bool use_stream_path(int M, int d, int r, int L, const DevInfo& di) {
@@ -477,6 +502,16 @@ int dlrb200_query(int M, int d, int r, int L, dlrb200_plan* plan) {
     return DLRB200_OK;
 }
 
+int dlrb200_query_call(int M, int d, int r, int L, dlrb200_plan* plan) {
+    const int rc = dlrb200_query(M, d, r, L, plan);
+    if (rc != DLRB200_OK || M == 0) return rc;
+    DevInfo di;
+    if (device_info(&di) != DLRB200_OK) return DLRB200_ERR_CUDA;
+    dlrb200_plan resident = *plan;
+    if (use_resident(M, d, r, L, di, &resident)) *plan = resident;
+    return DLRB200_OK;
+}
+
 int dlrb200_forward(const void* x, void* y, const void* Vp, const void* Up, int M, int d, int r, int L,
                     float eps, void* workspace, size_t workspace_bytes, int* status_dev, void* stream) {
     int rc = check_shape(M, d, r, L);
@@ -492,6 +527,14 @@ int dlrb200_forward(const void* x, void* y, const void* Vp, const void* Up, int 
     if (rc != DLRB200_OK) return rc;
     if (di.cc_major != 10) return DLRB200_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (use_resident(M, d, r, L, di)) {
+        EncodeTiledFn enc = encode_fn();
+        if (!enc) return DLRB200_ERR_CUDA;
+        rc = dlr::resident_forward(reinterpret_cast<void*>(enc), x, y, Vp, Up, M, d, r, L, eps, status_dev, st, di.smem_optin,
+                                   spin_limit());
+        if (rc == DLRB200_ERR_CUDA) g_last_cuda_error = int(cudaGetLastError());
+        return rc;
+    }
     if (use_pair_path(M, d, r, L, di) && dlr::stream_aligned(x, y)) {
         EncodeTiledFn enc = encode_fn();
         if (!enc) return DLRB200_ERR_CUDA;

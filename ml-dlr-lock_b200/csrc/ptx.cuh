@@ -111,6 +111,29 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
     return false;
 }
 
+// Bounded wait for a whole warp on one barrier, given up early once the word at `flag` (shared memory of this CTA) is
+// non-zero.  One block of assembly with uniform branches: every lane polls the same word, so the warp never splits, and
+// a look at a phase that is already complete costs about 60 cycles against 100 for the same loop in C++ (measured; the
+// difference is the bookkeeping for lanes that leave a loop at different times).  `limit` must not be 0.
+#define DLR_MBAR_WAIT_FLAG(NAME, FORM)                                                                              \
+    __device__ __forceinline__ bool NAME(uint32_t bar, uint32_t parity, uint32_t flag, uint32_t limit) {            \
+        uint32_t ok;                                                                                                \
+        asm volatile(                                                                                               \
+            "{\n\t.reg .pred P1, P2;\n\t.reg .u32 n, f;\n\tmov.u32 n, %4;\n"                                          \
+            "DLR_WAIT_%=:\n\t" FORM " P1, [%1], %2;\n\t@P1 bra.uni DLR_DONE_%=;\n\t"                                  \
+            "ld.volatile.shared.u32 f, [%3];\n\tsub.u32 n, n, 1;\n\tsetp.ne.u32 P2, n, 0;\n\t"                      \
+            "setp.eq.and.u32 P2, f, 0, P2;\n\t@P2 bra.uni DLR_WAIT_%=;\n"                                            \
+            "DLR_DONE_%=:\n\tselp.u32 %0, 1, 0, P1;\n\t}"                                                           \
+            : "=r"(ok)                                                                                              \
+            : "r"(bar), "r"(parity), "r"(flag), "r"(limit)                                                          \
+            : "memory");                                                                                            \
+        return ok != 0;                                                                                             \
+    }
+DLR_MBAR_WAIT_FLAG(mbar_wait_flag, "mbarrier.try_wait.parity.shared::cta.b64")
+// ... acquiring at cluster scope, for arrivals and stores that come from other CTAs
+DLR_MBAR_WAIT_FLAG(mbar_wait_flag_cluster, "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64")
+#undef DLR_MBAR_WAIT_FLAG
+
 // Polls granted to the waits that run only when a kernel is giving up: copies and
 // tensor-core work already requested must finish before the CTA leaves (they write
 // into its shared memory), whatever limit the caller set for the ordinary waits.

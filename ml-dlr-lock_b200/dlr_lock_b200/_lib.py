@@ -34,6 +34,7 @@ SIGNATURES = {
     "dlrb200_last_cuda_error": (_i, []),
     "dlrb200_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "dlrb200_query": (_i, [_i, _i, _i, _i, ctypes.POINTER(Plan)]),
+    "dlrb200_query_call": (_i, [_i, _i, _i, _i, ctypes.POINTER(Plan)]),
     "dlrb200_forward": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _vp, _sz, _vp, _vp]),
     "dlrb200_forward_host": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _vp, _sz, _vp, _vp]),
     "dlrb200_fold_weights": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),

@@ -3,7 +3,7 @@
 ``B_hi``, ``kernel``, ``callable`` (importable dotted path), ``config`` and
 ``note``.  This build has one backend behind one callable; it covers every batch
 size of all four model shapes.  The library picks among its device paths per
-call (``dlrb200_query`` reports the choice for a shape on the current device);
+call (``dlrb200_query_call`` reports the choice for a shape on the current device);
 the ranges below name the path that serves most of each range on a B200, and
 ``describe`` fills an entry from the library's own answer.
 """
@@ -18,7 +18,7 @@ MODEL_CONFIGS = {  # kernels/reference.py:18-23
 _CALLABLE = "dlr_lock_b200.ops.forward_xvu"
 
 PATH_NAMES = {1: "b200_striped", 2: "b200_cluster", 3: "b200_cluster_small", 4: "b200_streamed",
-              5: "b200_streamed_pairs", 6: "b200_striped_clusters"}
+              5: "b200_streamed_pairs", 6: "b200_striped_clusters", 7: "b200_resident"}
 PATH_CONFIGS = {
     1: "width-striped cooperative grid, TMA weight ring, one exchange per layer through L2",
     2: "128-row tiles on clusters of d/512 CTAs, activations resident in tensor memory, tcgen05",
@@ -27,12 +27,13 @@ PATH_CONFIGS = {
     5: "256-row tiles on CTA pairs (tcgen05 cta_group::2), activations streamed, exchange in distributed shared memory",
     6: "width-striped cooperative grid in clusters of 8: reduction inside a cluster in distributed shared memory, "
        "cluster sums through counted words in L2",
+    7: "clusters of 4/8/16 CTAs that keep a few rows each in registers, exchange in distributed shared memory",
 }
 
 
 def _entry(lo, hi, path, note):
     return {"B_lo": lo, "B_hi": hi, "kernel": PATH_NAMES[path], "callable": _CALLABLE,
-            "config": PATH_CONFIGS[path] + "; picked per call by dlrb200_query", "note": note}
+            "config": PATH_CONFIGS[path] + "; picked per call by dlrb200_query_call", "note": note}
 
 
 def _entries(name):
@@ -70,7 +71,7 @@ def describe(model: str, batch_size: int, depth: int):
     if entry is None:
         return None
     cfg = MODEL_CONFIGS[model]
-    plan = ops.query(batch_size, cfg["d"], cfg["r"], depth)
+    plan = ops.query_call(batch_size, cfg["d"], cfg["r"], depth)
     out = dict(entry)
     out["kernel"] = PATH_NAMES.get(plan.path, f"path{plan.path}")
     out["config"] = (f"{PATH_CONFIGS.get(plan.path, '')}; grid {plan.grid}, cluster {plan.cluster}, "
