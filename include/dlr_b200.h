@@ -147,6 +147,12 @@ DLRB200_API int dlrb200_forward_host(const void* x_host, void* y_host, void* x_d
  * unbounded. */
 DLRB200_API int dlrb200_status_to_host(const int* status_dev, int* status_host, void* stream);
 
+/* From now on a kernel that reports into status_dev also writes the word to
+ * status_host (pinned host memory), where the host sees it without any copy
+ * on the stream.  Null takes the mirror away; take it away before freeing
+ * either word.  The host sets both words back to 0 after reading. */
+DLRB200_API int dlrb200_set_status_mirror(const int* status_dev, int* status_host);
+
 /* Fold the per-layer gain into V and the ReZero scalar into U and stack the
  * result in the layouts dlrb200_forward takes.
  *   V (L, r, d), U (L, d, r), gain (L, d): bf16 device buffers; alpha (L) fp32.
@@ -154,6 +160,15 @@ DLRB200_API int dlrb200_status_to_host(const int* status_dev, int* status_host, 
  * Products are formed in fp32 and rounded once to bf16. */
 DLRB200_API int dlrb200_fold_weights(const void* V, const void* U, const void* gain, const float* alpha, void* Vp,
                          void* Up, int d, int r, int L, void* stream);
+
+/* The same for parameters that are not stacked: V, U, gain and alpha are HOST
+ * arrays of L device addresses, one tensor per layer ((r,d), (d,r), (d,) and
+ * one scale).  Without flags all are bf16. */
+#define DLRB200_FOLD_MATRICES_F32 1 /* V, U and the gains are fp32: rounded to bf16 first */
+#define DLRB200_FOLD_ALPHA_F32 2    /* the scales are fp32 */
+#define DLRB200_FOLD_ROUND_ALPHA 4  /* fp32 scales are rounded to bf16 first */
+DLRB200_API int dlrb200_fold_layers(const void* const* V, const void* const* U, const void* const* gain,
+                         const void* const* alpha, int flags, void* Vp, void* Up, int d, int r, int L, void* stream);
 
 /* Transpose a stack of L bf16 matrices (rows, cols) -> (cols, rows) on the
  * device; used to accept the reference CUDA convention Us (L, r, d). */

@@ -3,11 +3,14 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <shared_mutex>
+#include <vector>
 
 #include "cluster.h"
 #include "decode.h"
 #include "decode_cluster.h"
 #include "decode_tl.h"
+#include "fold.h"
 #include "resident.h"
 #include "stream.h"
 #include "stream_pair.h"
@@ -131,6 +134,7 @@ int striped_forward(const void* x, void* y, const void* Vp, const void* Up, int 
     a.p.counter = reinterpret_cast<unsigned int*>(ws);
     a.p.zacc = reinterpret_cast<float*>(ws + kCtrlBytes);
     a.p.status = status_dev;
+    a.p.mirror = dlr::status_mirror(status_dev);
     a.p.spin_limit = spin_limit();
 
     const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
@@ -167,6 +171,7 @@ int striped_tl_launch(const void* x, void* y, const void* Vp, const void* Up, in
     a.stream = stream;
     a.p.M = M; a.p.d = d; a.p.L = L; a.p.eps = eps; a.p.inv_d = 1.0f / float(d);
     a.p.status = status_dev;
+    a.p.mirror = dlr::status_mirror(status_dev);
     a.p.spin_limit = spin_limit();
     if (plan_only) return dlr::decode_tl_launch(a, plan_only);
     EncodeTiledFn enc = encode_fn();
@@ -189,23 +194,6 @@ int striped_tl_launch(const void* x, void* y, const void* Vp, const void* Up, in
     const int rc = dlr::decode_tl_launch(a, nullptr);
     if (rc == DLRB200_ERR_CUDA) g_last_cuda_error = int(cudaGetLastError());
     return rc;
-}
-
-__global__ void fold_v_kernel(const __nv_bfloat16* __restrict__ V, const __nv_bfloat16* __restrict__ gain,
-                              __nv_bfloat16* __restrict__ Vp, int d, int r, size_t total) {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const size_t layer = i / (size_t(r) * d);
-    const int col = int(i % d);
-    Vp[i] = __float2bfloat16_rn(__bfloat162float(V[i]) * __bfloat162float(gain[layer * d + col]));
-}
-
-__global__ void fold_u_kernel(const __nv_bfloat16* __restrict__ U, const float* __restrict__ alpha,
-                              __nv_bfloat16* __restrict__ Up, int d, int r, size_t total) {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const size_t layer = i / (size_t(r) * d);
-    Up[i] = __float2bfloat16_rn(__bfloat162float(U[i]) * alpha[layer]);
 }
 
 __global__ void transpose_stack_kernel(const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ dst,
@@ -418,6 +406,18 @@ bool use_striped_clusters(int M, int d, int r, int L, const DevInfo& di) {
 
 namespace dlr {
 
+// (status word, host copy) pairs: one per stream a process uses
+struct Mirror { const int* status; int* host; };
+static std::vector<Mirror> g_mirrors;
+static std::shared_mutex g_mirrors_mutex;
+
+int* status_mirror(const int* status_dev) {
+    std::shared_lock<std::shared_mutex> lock(g_mirrors_mutex);
+    for (const Mirror& m : g_mirrors)
+        if (m.status == status_dev) return m.host;
+    return nullptr;
+}
+
 bool encode_2d_bf16(void* encode_fn_ptr, CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
                     int box_inner, int box_outer, int swizzle_bytes) {
     EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(encode_fn_ptr);
@@ -605,18 +605,41 @@ int dlrb200_status_to_host(const int* status_dev, int* status_host, void* stream
                : DLRB200_ERR_CUDA;
 }
 
+int dlrb200_set_status_mirror(const int* status_dev, int* status_host) {
+    if (!status_dev) return DLRB200_ERR_INVALID_ARG;
+    std::unique_lock<std::shared_mutex> lock(dlr::g_mirrors_mutex);
+    auto& all = dlr::g_mirrors;
+    for (size_t i = 0; i < all.size(); ++i)
+        if (all[i].status == status_dev) {
+            if (status_host) all[i].host = status_host;
+            else all.erase(all.begin() + i);
+            return DLRB200_OK;
+        }
+    if (status_host) all.push_back({status_dev, status_host});
+    return DLRB200_OK;
+}
+
 int dlrb200_fold_weights(const void* V, const void* U, const void* gain, const float* alpha, void* Vp,
                          void* Up, int d, int r, int L, void* stream) {
     if (!V || !U || !gain || !alpha || !Vp || !Up || d <= 0 || r <= 0 || L <= 0) return DLRB200_ERR_INVALID_ARG;
-    const size_t total = size_t(L) * r * d;
-    const int threads = 256;
-    const unsigned blocks = unsigned((total + threads - 1) / threads);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    fold_v_kernel<<<blocks, threads, 0, st>>>(static_cast<const __nv_bfloat16*>(V),
-                                              static_cast<const __nv_bfloat16*>(gain),
-                                              static_cast<__nv_bfloat16*>(Vp), d, r, total);
-    fold_u_kernel<<<blocks, threads, 0, st>>>(static_cast<const __nv_bfloat16*>(U), alpha,
-                                              static_cast<__nv_bfloat16*>(Up), d, r, total);
+    const size_t n = size_t(r) * d;
+    std::vector<const void*> at(size_t(4) * L);
+    for (int l = 0; l < L; ++l) {
+        at[l] = static_cast<const __nv_bfloat16*>(V) + l * n;
+        at[L + l] = static_cast<const __nv_bfloat16*>(U) + l * n;
+        at[2 * L + l] = static_cast<const __nv_bfloat16*>(gain) + size_t(l) * d;
+        at[3 * L + l] = alpha + l;
+    }
+    return dlrb200_fold_layers(at.data(), at.data() + L, at.data() + 2 * L, at.data() + 3 * L, DLRB200_FOLD_ALPHA_F32, Vp, Up, d, r, L,
+                               stream);
+}
+
+int dlrb200_fold_layers(const void* const* V, const void* const* U, const void* const* gain, const void* const* alpha,
+                        int flags, void* Vp, void* Up, int d, int r, int L, void* stream) {
+    if (!V || !U || !gain || !alpha || !Vp || !Up || d <= 0 || r <= 0 || L <= 0) return DLRB200_ERR_INVALID_ARG;
+    if (!dlr::fold_layers(V, U, gain, alpha, (flags & DLRB200_FOLD_MATRICES_F32) != 0, (flags & DLRB200_FOLD_ALPHA_F32) != 0,
+                          (flags & DLRB200_FOLD_ROUND_ALPHA) != 0, Vp, Up, d, r, L, static_cast<cudaStream_t>(stream)))
+        return DLRB200_ERR_UNSUPPORTED_SHAPE;
     return cuda_ok(cudaGetLastError()) ? DLRB200_OK : DLRB200_ERR_CUDA;
 }
 

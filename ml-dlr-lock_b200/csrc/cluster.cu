@@ -71,6 +71,7 @@ struct ClusterParams {
     int M, d, L;
     float eps, inv_d;
     int* status;
+    int* mirror;                // host copy of the status word, or null
     unsigned int spin_limit;
     int stages;
     int num_tiles;
@@ -496,7 +497,7 @@ dlr_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constan
 
     if (err) {
         *abort_flag = 1;
-        atomicCAS(p.status, 0, err | (err_layer << 8));
+        report_status(p.status, p.mirror, err | (err_layer << 8));
     }
     __syncwarp();
     tc_fence_before();
@@ -561,6 +562,7 @@ int launch_cluster(void* enc, const void* x, void* y, const void* Vp, const void
     p.y = static_cast<__nv_bfloat16*>(y);
     p.M = M; p.d = d; p.L = L; p.eps = eps; p.inv_d = 1.0f / float(d);
     p.status = status_dev;
+    p.mirror = status_mirror(status_dev);
     p.spin_limit = spin_limit;
     p.stages = stages;
     p.num_tiles = num_tiles;

@@ -15,6 +15,9 @@ namespace dlr {
 bool encode_2d_bf16(void* encode_fn_ptr, CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
                     int box_inner, int box_outer, int swizzle_bytes);
 
+// Host address that kernels given `status_dev` also report to (dlrb200_set_status_mirror), or null.
+int* status_mirror(const int* status_dev);
+
 bool cluster_supported(int d, int r, int L);
 size_t cluster_workspace_bytes(int M, int d, int r, int L);
 int cluster_plan(int M, int d, int r, int L, int num_sms, int smem_optin, dlrb200_plan* plan);

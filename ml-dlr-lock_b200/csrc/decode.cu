@@ -486,7 +486,7 @@ dlr_decode_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant
         // Give up: record why and where, then wait (bounded) for the copies
         // still in flight into this CTA's shared memory before leaving.
         if (tid == 0) {
-            atomicCAS(p.status, 0, err | (l << 8));
+            report_status(p.status, p.mirror, err | (l << 8));
             const int hi = (l + S < p.L) ? l + S : p.L;
             const int lo = (err == DLRB200_ERR_TIMEOUT_COPY || nothing_consumed) ? l : l + 1;
             for (int j = lo; j < hi; ++j) mbar_wait(smem_u32(&full[j % S]), (j / S) & 1, kDrainPolls);

@@ -21,6 +21,7 @@ struct DecodeParams {
     float* zacc;              // 3 slots x 64 rows x (r+4) floats, zero on entry
     unsigned int* counter;    // zero on entry
     int* status;              // device status word, untouched unless a wait gives up
+    int* mirror;              // host copy of the status word, or null
     unsigned int spin_limit;
     int stages;               // filled by the launcher
 };

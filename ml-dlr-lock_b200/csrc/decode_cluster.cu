@@ -56,6 +56,7 @@ struct DCParams {
     int M, d, L;
     float eps, inv_d;
     int* status;
+    int* mirror;                // host copy of the status word, or null
     unsigned int spin_limit;
     int stages;
     int cs;
@@ -229,7 +230,7 @@ dlr_decode_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_
             if (err) {
                 if (!*abort_flag) {
                     *abort_flag = 1;
-                    atomicCAS(p.status, 0, err | (l << 8));
+                    report_status(p.status, p.mirror, err | (l << 8));
                 }
                 // tiles already requested still land in this CTA's ring: wait (bounded) before leaving.  A group
                 // cut short by the error never completes its byte count; older groups have been consumed.
@@ -404,7 +405,7 @@ dlr_decode_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_
         if (p.prof && tid == 0 && blockIdx.x == 0)
             for (int k = 0; k < 8; ++k) p.prof[k] = (unsigned long long)pc[k];
         if (err) {
-            if (tid == 0) atomicCAS(p.status, 0, err | (l << 8));
+            if (tid == 0) report_status(p.status, p.mirror, err | (l << 8));
         } else {
             if (rows > 0) p.y[size_t(row0) * p.d + stripe0 + tid] = __float2bfloat16_rn(h0);
             if (rows > 1) p.y[size_t(row0 + 1) * p.d + stripe0 + tid] = __float2bfloat16_rn(h1);
@@ -465,6 +466,7 @@ int launch_dc(void* enc, const void* x, void* y, const void* Vp, const void* Up,
     p.y = static_cast<__nv_bfloat16*>(y);
     p.M = M; p.d = d; p.L = L; p.eps = eps; p.inv_d = 1.0f / float(d);
     p.status = status_dev;
+    p.mirror = status_mirror(status_dev);
     p.spin_limit = spin_limit;
     p.stages = stages;
     p.cs = cs;

@@ -23,6 +23,7 @@ struct DecodeTLParams {
     float* pre;                   // [CTAs][64] sums of squares of the input per CTA
     unsigned int* counter;        // zero on entry
     int* status;                  // device status word, untouched unless a wait gives up
+    int* mirror;              // host copy of the status word, or null
     unsigned int spin_limit;
     int stages;                   // filled by the launcher
 };

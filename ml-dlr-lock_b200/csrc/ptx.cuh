@@ -159,6 +159,14 @@ struct RingPos {
     }
 };
 
+// A wait has given up: the first report stays in the status word, and goes to the host's copy of it if there is one.
+__device__ __forceinline__ void report_status(int* status, int* mirror, int word) {
+    if (atomicCAS(status, 0, word) == 0 && mirror != nullptr) {
+        *reinterpret_cast<volatile int*>(mirror) = word;
+        __threadfence_system();
+    }
+}
+
 // ---------------------------------------------------------------------------
 // proxy fences
 // ---------------------------------------------------------------------------

@@ -53,6 +53,7 @@ struct RParams {
     int rows_per_cluster;
     float eps, inv_d;
     int* status;
+    int* mirror;                // host copy of the status word, or null
     unsigned int spin_limit;
 };
 
@@ -102,7 +103,7 @@ struct RBars {
     uint64_t rbar[2];          // partial z and sums of squares have arrived (bytes); BC: by parity of the layer
     uint64_t sbar;             // RS: s has arrived (bytes)
     int fail[2];               // by parity of the layer: a warp gave up before this layer's block barrier
-    int abort_flag;
+    int abort_flag, give_up;
 };
 static_assert(sizeof(RBars) <= 1024, "barrier block");
 
@@ -164,10 +165,9 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             mbar_init(smem_u32(&bars->rbar[b]), 1);
         }
         mbar_init(smem_u32(&bars->sbar), 1);
-        // a status word that is set already: every warp leaves its loop in the first layer
-        const int set = *reinterpret_cast<volatile int*>(p.status) != 0;
-        fail[0] = fail[1] = set;
-        *abort_flag = set;
+        fail[0] = fail[1] = 0;
+        *abort_flag = 0;
+        bars->give_up = 0;
         fence_mbar_init();
         tma_prefetch_desc(&tmV);
         tma_prefetch_desc(&tmU);
@@ -397,6 +397,8 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             for (l = 0; l < p.L && !err; ++l) {
                 for (int s = 0; s < C::NVS; ++s) ask_v();
                 for (int s = 0; s < C::NUS; ++s) ask_u();
+                // the status word was set before this launch: give up
+                if (l == 0 && *reinterpret_cast<volatile int*>(p.status) != 0) *reinterpret_cast<volatile int*>(&bars->give_up) = 1;
             }
             if (err || *abort_flag) drain_copies();
         }
@@ -494,6 +496,7 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             if (warp == NU - 1 && lane == 0) {
                 mbar_arrive_expect_tx(rbar_s, z_bytes + uint32_t(CS * 4 * rows));
                 if (!BC) mbar_arrive_expect_tx(sbar_s, uint32_t(rows * R * 2));
+                if (*reinterpret_cast<volatile int*>(&bars->give_up)) err = DLRB200_ERR_TIMEOUT_BARRIER;
             }
             // ---- this layer's U' fragments, while the V warps work and the partials travel
             if constexpr (C::PREF) {
@@ -663,7 +666,7 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
     }
     if (err) {
         *abort_flag = 1;
-        atomicCAS(p.status, 0, err | ((l & 0xffff) << 8));
+        report_status(p.status, p.mirror, err | ((l & 0xffff) << 8));
     }
     __syncwarp();
     __syncthreads();
@@ -777,6 +780,7 @@ struct RLaunch {
         p.rows_per_cluster = sh.rows;
         p.eps = a.eps; p.inv_d = 1.0f / float(a.d);
         p.status = a.status;
+        p.mirror = status_mirror(a.status);
         p.spin_limit = a.spin_limit > 8 ? a.spin_limit >> 3 : 1;
         CUtensorMap tmV, tmU;
         if (!encode_2d_bf16(a.enc, &tmV, a.Vp, uint64_t(a.d), uint64_t(a.L) * R, 64, R, 128) ||

@@ -52,6 +52,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "cluster.h"
 #include "ptx.cuh"
 #include "stream.h"
 
@@ -125,6 +126,7 @@ struct SParams {
     uint4* xchg;              // sp > 1: per-layer exchange of the partial z between the CTAs of a cluster
     float eps, inv_d;
     int* status;
+    int* mirror;                // host copy of the status word, or null
     unsigned int spin_limit;
     unsigned long long* prof; // optional cycle counters (debug), or null
 };
@@ -644,7 +646,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     if (err) {
         if (!*abort_flag) {
             *abort_flag = 1;
-            atomicCAS(p.status, 0, err | ((err_layer & 0xffff) << 8));
+            report_status(p.status, p.mirror, err | ((err_layer & 0xffff) << 8));
         }
     }
     __syncwarp();
@@ -741,6 +743,7 @@ int launch_stream(void* enc, const void* x, void* y, const void* Vp, const void*
     p.eps = eps;
     p.inv_d = 1.0f / float(d);
     p.status = status_dev;
+    p.mirror = status_mirror(status_dev);
     p.spin_limit = spin_limit;
     p.prof = prof;
     const cudaError_t ce = cudaLaunchKernelEx(&cfg, kern, tmX, tmY, tmV, tmU, p);

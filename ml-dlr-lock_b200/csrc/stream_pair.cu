@@ -44,6 +44,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "cluster.h"
 #include "ptx.cuh"
 #include "stream_pair.h"
 
@@ -122,6 +123,7 @@ struct PParams {
     int num_tiles;            // 256-row tiles
     float eps, inv_d;
     int* status;
+    int* mirror;                // host copy of the status word, or null
     unsigned int spin_limit;
     unsigned long long* prof; // time stamps (profiling instantiation), or null
     int trace_layer;
@@ -674,7 +676,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     if (err) {
         if (!*abort_flag) {
             *abort_flag = 1;
-            atomicCAS(p.status, 0, err | ((err_layer & 0xffff) << 8));
+            report_status(p.status, p.mirror, err | ((err_layer & 0xffff) << 8));
         }
     }
     __syncwarp();
@@ -799,6 +801,7 @@ int launch_pair(void* enc, const void* x, void* y, const void* Vp, const void* U
     p.eps = eps;
     p.inv_d = 1.0f / float(d);
     p.status = status_dev;
+    p.mirror = status_mirror(status_dev);
     p.spin_limit = spin_limit;
     p.prof = prof;
     p.trace_layer = L / 2;

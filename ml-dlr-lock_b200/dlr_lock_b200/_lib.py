@@ -38,8 +38,10 @@ SIGNATURES = {
     "dlrb200_forward": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _vp, _sz, _vp, _vp]),
     "dlrb200_forward_host": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _vp, _sz, _vp, _vp]),
     "dlrb200_fold_weights": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp]),
+    "dlrb200_fold_layers": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _i, _vp]),
     "dlrb200_transpose_stack": (_i, [_vp, _vp, _i, _i, _i, _vp]),
     "dlrb200_status_to_host": (_i, [_vp, _vp, _vp]),
+    "dlrb200_set_status_mirror": (_i, [_vp, _vp]),
     "dlrb200_forward_static": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _f, _vp, _vp]),
 }
 
@@ -74,6 +76,27 @@ def load() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+_host_module = None
+
+
+def host():
+    """The native host helper ``_host`` (csrc/host.cpp), loaded once."""
+    global _host_module
+    if _host_module is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries, which the helper links against)
+
+        path = os.path.join(HERE, "_host.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `python -m dlr_lock_b200.build`.")
+        spec = importlib.util.spec_from_file_location("_host", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _host_module = mod
+    return _host_module
 
 
 def strerror(code: int) -> str:

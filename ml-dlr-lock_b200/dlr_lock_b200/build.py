@@ -6,6 +6,8 @@ Every ``.cu`` under ``csrc/`` is compiled with
 ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` and linked into
 ``libdlr_b200.so`` next to this file.  The CUDA runtime is linked statically,
 so the library does not depend on which runtime the host process loaded.
+``csrc/host.cpp`` becomes the Python module ``_host`` (walks over a net's
+parameters; see there).
 """
 from __future__ import annotations
 
@@ -19,6 +21,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.normpath(os.path.join(HERE, "..", "csrc"))
 INCLUDE = os.path.normpath(os.path.join(HERE, "..", "..", "include"))
 LIB_PATH = os.path.join(HERE, "libdlr_b200.so")
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_PATH = os.path.join(HERE, "_host.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 NVCC_FLAGS = [
@@ -46,8 +50,31 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_host(force: bool = False) -> str:
+    """Compile the host-side helper module ``_host`` against torch's headers, if it is out of date."""
+    if not force and not _stale(HOST_PATH, [HOST_SRC]):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", sysconfig.get_paths()["include"]]
+    for p in include_paths():
+        cmd += ["-isystem", p]
+    cmd += [HOST_SRC, "-o", HOST_PATH]
+    for p in library_paths():
+        cmd += ["-L", p]
+    r = subprocess.run(cmd + ["-ltorch_python", "-ltorch_cpu", "-lc10"], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return HOST_PATH
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compile what is out of date and return the path of the shared library."""
+    """Compile what is out of date (the CUDA library and the host helper) and return the path of the shared library."""
+    build_host(force)
     os.makedirs(OBJ_DIR, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(INCLUDE, "dlr_b200.h"))

@@ -22,7 +22,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.utils.checkpoint import checkpoint as _checkpoint
 
-from . import ops
+from . import _lib, ops
 
 
 def dlrnet_param_count(d: int, r: int, depth: int) -> int:
@@ -88,15 +88,15 @@ class DLRNet(nn.Module):
         return self
 
     # ---- derived folded weights ----------------------------------------------
+    def _param_dicts(self):
+        """The parameters as four dicts (V, U, gains, alphas), layer by layer."""
+        return tuple(p._parameters if isinstance(p, nn.ParameterList) else {str(i): t for i, t in enumerate(p)}
+                     for p in (self.Vs, self.Us, self.rms_w, self.alphas))
+
     def _cache_key(self):
         # every parameter of every layer: storage address and in-place version counter.  A write through
         # ``p.data`` (``p.data.copy_(...)``) bumps neither: call ``invalidate()`` after such an edit.
-        key = []
-        for plist in (self.Vs, self.Us, self.rms_w, self.alphas):
-            for p in plist:
-                key.append(p.data_ptr())
-                key.append(p._version)
-        return tuple(key)
+        return _lib.host().snapshot(self._param_dicts())
 
     def invalidate(self):
         """Drop the folded weights; they are rebuilt on the next fast forward.  Needed after writes
@@ -105,14 +105,15 @@ class DLRNet(nn.Module):
 
     def folded_weights(self):
         """(V' (L,r,d), U' (L,d,r)) bf16 on the parameters' device, cached."""
-        key = self._cache_key()
-        if self._folded is None or self._folded[0] != key:
-            V = torch.stack([p.detach() for p in self.Vs])
-            U = torch.stack([p.detach() for p in self.Us])
-            w = torch.stack([p.detach() for p in self.rms_w])
-            a = torch.stack([p.detach() for p in self.alphas])
-            Vp, Up = ops.fold_weights(V, U, w, a)
-            self._folded = (key, Vp, Up)
+        dicts, host = self._param_dicts(), _lib.host()
+        if self._folded is None or not host.unchanged(self._folded[0], dicts):
+            found = host.layers(dicts)
+            if found is not None:
+                Vp, Up = ops.fold_layers(found, round_alpha=False)
+            else:
+                V, U, w, a = (torch.stack([p.detach() for p in d.values()]) for d in dicts)
+                Vp, Up = ops.fold_weights(V, U, w, a)
+            self._folded = (host.snapshot(dicts), Vp, Up)
         return self._folded[1], self._folded[2]
 
     def _load_from_state_dict(self, *args, **kwargs):

@@ -23,74 +23,76 @@ from . import _lib
 EPS = 1e-6
 
 class _Scratch:
-    """Per (device, stream): workspace, device status word and its pinned host mirror."""
+    """Per (device, stream): workspace, device status word and its mirror in pinned host memory.
 
-    __slots__ = ("ws", "status", "status_host", "retired")
+    A kernel writes both words, and only when a device-side wait gives up; the host looks at the mirror without a copy or a
+    synchronisation.
+    """
+
+    __slots__ = ("ws", "nbytes", "ptr", "status", "status_ptr", "mirror", "word", "retired")
 
     def __init__(self, device: torch.device, nbytes: int):
-        self.ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
-        self.status_host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.status_ptr = self.status.data_ptr()
+        self.mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.word = ctypes.c_int.from_address(self.mirror.data_ptr())
+        _lib.check(_lib.load().dlrb200_set_status_mirror(self.status_ptr, self.mirror.data_ptr()), "dlrb200_set_status_mirror")
         # workspaces that were outgrown: a CUDA graph captured earlier has their address in its nodes, so
         # they stay allocated for the life of the process (they are small: at most a few tens of MB)
         self.retired = []
+        self.ws = None
+        self.resize(device, nbytes)
+
+    def resize(self, device: torch.device, nbytes: int):
+        if self.ws is not None:
+            self.retired.append(self.ws)
+        self.ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        self.nbytes = nbytes
+        self.ptr = self.ws.data_ptr()
 
 
 _workspaces: Dict[Tuple[int, int], _Scratch] = {}
 _derived: Dict[Tuple, Tuple[torch.Tensor, ...]] = {}
 _MIN_WORKSPACE = 1 << 20
+# the current stream of a device as an address, without building a stream object
+_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else None
 
 
-def _ptr(t: torch.Tensor) -> ctypes.c_void_p:
-    return ctypes.c_void_p(t.data_ptr())
-
-
-def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream_ptr(index: int) -> int:
+    return _raw_stream(index)
 
 
 def _raise_status(ent: _Scratch, word: int):
-    ent.status_host.zero_()
-    ent.status.zero_()          # a non-zero word makes later calls give up early: clear it before reporting
+    ent.word.value = 0          # a non-zero word makes later calls give up early: clear it before reporting
+    ent.status.zero_()
     raise _lib.DlrB200Error(word & 0xff, f"device status: {_lib.strerror(word & 0xff)} at layer {word >> 8}")
 
 
-def _workspace(device: torch.device, nbytes: int) -> _Scratch:
-    """Scratch + status word for the current (device, stream); grown on demand.
+def _workspace(index: int, stream: int, nbytes: int) -> _Scratch:
+    """Scratch + status word for a (device, stream); grown on demand.
 
     One workspace per stream, because calls that share one must not overlap.  A workspace that is outgrown
     is kept, not freed: a CUDA graph captured while it was current still clears and uses that memory on
-    every replay.  Also the lazy error check: the status word of the calls before, mirrored to pinned host
-    memory by a copy on the stream after every forward, is looked at here without synchronising.
+    every replay.  Also the lazy error check: a wait that gave up in a call before, on this stream, is
+    reported here without synchronising.
     """
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
-    ent = _workspaces.get(key)
+    ent = _workspaces.get((index, stream))
     if ent is None:
-        ent = _Scratch(device, max(nbytes, _MIN_WORKSPACE))
-        _workspaces[key] = ent
-    else:
-        word = int(ent.status_host[0])
-        if word != 0 and not torch.cuda.is_current_stream_capturing():
-            _raise_status(ent, word)
-        if ent.ws.numel() < nbytes:
-            ent.retired.append(ent.ws)
-            ent.ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        ent = _workspaces[(index, stream)] = _Scratch(torch.device("cuda", index), max(nbytes, _MIN_WORKSPACE))
+        return ent
+    word = ent.word.value
+    if word != 0 and not torch.cuda.is_current_stream_capturing():
+        _raise_status(ent, word)
+    if ent.nbytes < nbytes:
+        ent.resize(torch.device("cuda", index), nbytes)
     return ent
-
-
-def _mirror_status(lib, ent: _Scratch, device: torch.device) -> None:
-    """Queue the 4-byte copy of the status word to its pinned host mirror behind the forward."""
-    rc = lib.dlrb200_status_to_host(_ptr(ent.status), ctypes.c_void_p(ent.status_host.data_ptr()),
-                                    _stream_ptr(device))
-    _lib.check(rc, "dlrb200_status_to_host")
 
 
 def check_status(device=None) -> None:
     """Synchronise and raise if a bounded device-side wait gave up on `device`.
 
-    Without this call a timeout still surfaces, one call late: every forward mirrors the status word to
-    pinned host memory on its stream, and the next forward on that stream looks at the mirror first.
+    Without this call a timeout still surfaces, one call late: the next forward on that stream looks at the
+    status word first.
     """
     for (dev, _), ent in list(_workspaces.items()):
         if device is not None and torch.device(device).index not in (None, dev):
@@ -108,7 +110,7 @@ def _check_inputs(x, Vp, Up):
     if Vp.dim() != 3 or Up.dim() != 3:
         raise ValueError("folded weights must be V' (L,r,d) and U' (L,d,r)")
     L, r, d = Vp.shape
-    if tuple(Up.shape) != (L, d, r):
+    if Up.shape != (L, d, r):
         raise ValueError(f"U' has shape {tuple(Up.shape)}, expected {(L, d, r)}")
     if x.shape[-1] != d:
         raise ValueError(f"last dimension of x is {x.shape[-1]}, expected d={d}")
@@ -126,24 +128,26 @@ def forward_folded(x: torch.Tensor, Vp: torch.Tensor, Up: torch.Tensor, eps: flo
     next forward on the same stream that runs after the failed one has finished.
     """
     L, r, d = _check_inputs(x, Vp, Up)
-    lib = _lib.load()
-    x2 = x.reshape(-1, d)
-    if not x2.is_contiguous():
-        x2 = x2.contiguous()
-    M = x2.shape[0]
-    y2 = torch.empty_like(x2) if out is None else out.view(-1, d)
-    if M == 0:
-        return y2.view(x.shape)
-    with torch.cuda.device(x.device):
+    index = x.get_device()
+    if index != torch.cuda.current_device():
+        with torch.cuda.device(index):
+            return forward_folded(x, Vp, Up, eps, out)
+    if not x.is_contiguous():
+        x = x.contiguous()
+    y = torch.empty_like(x) if out is None else out.view(-1, d)
+    M = x.numel() // d
+    if M != 0:
+        lib = _lib.load()
         need = lib.dlrb200_workspace_bytes(M, d, r, L)
         if need == 0:
             _lib.check(2, f"dlrb200_forward(M={M}, d={d}, r={r}, L={L})")
-        ent = _workspace(x.device, need)
-        rc = lib.dlrb200_forward(_ptr(x2), _ptr(y2), _ptr(Vp), _ptr(Up), M, d, r, L, float(eps),
-                                 _ptr(ent.ws), ent.ws.numel(), _ptr(ent.status), _stream_ptr(x.device))
-        _lib.check(rc, f"dlrb200_forward(M={M}, d={d}, r={r}, L={L})")
-        _mirror_status(lib, ent, x.device)
-    return y2.view(x.shape)
+        stream = _stream_ptr(index)
+        ent = _workspace(index, stream, need)
+        rc = lib.dlrb200_forward(x.data_ptr(), y.data_ptr(), Vp.data_ptr(), Up.data_ptr(), M, d, r, L, eps,
+                                 ent.ptr, ent.nbytes, ent.status_ptr, stream)
+        if rc != 0:
+            _lib.check(rc, f"dlrb200_forward(M={M}, d={d}, r={r}, L={L})")
+    return y if out is None else y.view(x.shape)
 
 
 def forward_host(x_host: torch.Tensor, y_host: torch.Tensor, x_dev: torch.Tensor, y_dev: torch.Tensor,
@@ -153,13 +157,13 @@ def forward_host(x_host: torch.Tensor, y_host: torch.Tensor, x_dev: torch.Tensor
     M = x_host.numel() // d
     lib = _lib.load()
     with torch.cuda.device(Vp.device):
+        index = Vp.get_device()
         need = lib.dlrb200_workspace_bytes(M, d, r, L)
-        ent = _workspace(Vp.device, need)
-        rc = lib.dlrb200_forward_host(_ptr(x_host), _ptr(y_host), _ptr(x_dev), _ptr(y_dev), _ptr(Vp), _ptr(Up),
-                                      M, d, r, L, float(eps), _ptr(ent.ws), ent.ws.numel(), _ptr(ent.status),
-                                      _stream_ptr(Vp.device))
+        stream = _stream_ptr(index)
+        ent = _workspace(index, stream, need)
+        rc = lib.dlrb200_forward_host(x_host.data_ptr(), y_host.data_ptr(), x_dev.data_ptr(), y_dev.data_ptr(), Vp.data_ptr(),
+                                      Up.data_ptr(), M, d, r, L, float(eps), ent.ptr, ent.nbytes, ent.status_ptr, stream)
         _lib.check(rc, "dlrb200_forward_host")
-        _mirror_status(lib, ent, Vp.device)
 
 
 def query(M: int, d: int, r: int, L: int) -> _lib.Plan:
@@ -194,9 +198,26 @@ def fold_weights(V: torch.Tensor, U: torch.Tensor, gain: torch.Tensor, alpha: to
     Vp = torch.empty_like(Vb)
     Up = torch.empty_like(Ub)
     with torch.cuda.device(V.device):
-        rc = _lib.load().dlrb200_fold_weights(_ptr(Vb), _ptr(Ub), _ptr(gb), _ptr(af), _ptr(Vp), _ptr(Up),
-                                              d, r, L, _stream_ptr(V.device))
+        rc = _lib.load().dlrb200_fold_weights(Vb.data_ptr(), Ub.data_ptr(), gb.data_ptr(), af.data_ptr(), Vp.data_ptr(),
+                                              Up.data_ptr(), d, r, L, _stream_ptr(V.get_device()))
     _lib.check(rc, "dlrb200_fold_weights")
+    return Vp, Up
+
+
+_MATRICES_F32, _ALPHA_F32, _ROUND_ALPHA = 1, 2, 4
+
+
+def fold_layers(found, round_alpha: bool):
+    """Folded stacks from unstacked parameters, as ``_host.layers`` or ``_host.state_layers`` found them: the tensors are read
+    where they are.  The same values as ``fold_weights``; ``round_alpha`` rounds fp32 scales to bf16 first."""
+    L, r, d, index, bf16, alpha_bf16, V, U, gain, alpha = found
+    flags = (0 if bf16 else _MATRICES_F32) | (0 if alpha_bf16 else _ALPHA_F32) | (_ROUND_ALPHA if round_alpha else 0)
+    device = torch.device("cuda", index)
+    Vp = torch.empty((L, r, d), dtype=torch.bfloat16, device=device)
+    Up = torch.empty((L, d, r), dtype=torch.bfloat16, device=device)
+    with torch.cuda.device(device):
+        rc = _lib.load().dlrb200_fold_layers(V, U, gain, alpha, flags, Vp.data_ptr(), Up.data_ptr(), d, r, L, _stream_ptr(index))
+    _lib.check(rc, "dlrb200_fold_layers")
     return Vp, Up
 
 
@@ -206,7 +227,7 @@ def transpose_stack(src: torch.Tensor) -> torch.Tensor:
     src = src.contiguous()
     dst = torch.empty((L, cols, rows), dtype=src.dtype, device=src.device)
     with torch.cuda.device(src.device):
-        rc = _lib.load().dlrb200_transpose_stack(_ptr(src), _ptr(dst), L, rows, cols, _stream_ptr(src.device))
+        rc = _lib.load().dlrb200_transpose_stack(src.data_ptr(), dst.data_ptr(), L, rows, cols, _stream_ptr(src.get_device()))
     _lib.check(rc, "dlrb200_transpose_stack")
     return dst
 

@@ -16,7 +16,7 @@ from typing import List, Optional
 
 import torch
 
-from . import ops
+from . import _lib, ops
 
 _KEY = re.compile(r"^(?:_orig_mod\.)?(Vs|Us|rms_w|alphas)\.(\d+)$")
 
@@ -52,6 +52,12 @@ def pack_state_dict(sd: dict, device, eps: float = 1e-6, dtype: torch.dtype = to
     them into a bf16 module (``replace_layer_mlp`` casts to the layer's dtype, dlr_lock/model.py:171-172)
     before its packer runs, so alpha reaches the fold as a bf16 value.  The result is then bit-identical to
     ``DLRNet.folded_weights()`` of a module loaded from the same file."""
+    device = torch.device(device)
+    if dtype == torch.bfloat16 and device.type == "cuda":
+        # complete layers on the device already: folded from where they are, without stacked copies
+        found = _lib.host().state_layers(sd)
+        if found is not None and found[3] == (torch.cuda.current_device() if device.index is None else device.index):
+            return PackedNet(*ops.fold_layers(found, round_alpha=True), eps)
     groups = {"Vs": {}, "Us": {}, "rms_w": {}, "alphas": {}}
     for k, v in sd.items():
         m = _KEY.match(k)
