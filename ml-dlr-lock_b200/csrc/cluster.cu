@@ -24,12 +24,11 @@
 // rounded to bf16 right after the sum anyway, and the end-to-end error is
 // unchanged by it.
 //
-// Two MMA warps.  One thread can issue a 128xNx16 tcgen05.mma only about every
-// 125 cycles for any N <= 128 (measured), half of what the tensor pipe executes
-// at N = 128, while two issuing warps run side by side at full rate.  So the V
-// contraction is split along K over two warps into the two accumulators (the
-// halves are added when z is read out), and the four 128-column chunks of the
-// U contraction alternate between the two warps and accumulators.
+// Two MMA warps.  The V contraction is split along K over two issuing warps into
+// the two accumulators (the halves are added when z is read out), and the four
+// 128-column chunks of the U contraction alternate between the two warps and
+// accumulators: a warp that waits for its accumulator or its weights does not
+// hold up the other.
 //
 // Exchange mechanics.  Every remote write is an asynchronous store
 // (st.async ... shared::cluster) whose bytes are counted on the RECEIVER's
@@ -124,7 +123,7 @@ dlr_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constan
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0);
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int cluster_id = blockIdx.x / CS;
@@ -209,7 +208,7 @@ dlr_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constan
         // =============================== MMA issuer b ===============================
         // b = 0: K tiles 0-3 of the V contraction, U chunks 0 and 2, accumulator 0
         // b = 1: K tiles 4-7,                       U chunks 1 and 3, accumulator 1
-        if (lane == 0) {
+        if (elect_one()) {
             const int b = warp - 1;
             const uint32_t acc = tmem_base + kAcc0 + uint32_t(b) * 128u;
             const uint32_t idesc_v = umma_idesc_bf16(128, R);

@@ -163,7 +163,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     volatile int* abort_flag = &bars->abort_flag;
     volatile unsigned int* stored = &bars->stored;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0);
     const int lane = threadIdx.x & 31;
     const Waiter w{abort_flag, p.spin_limit >> 2};
 
@@ -304,7 +304,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     } else if (warp == 1) {
         // =============================== U-MMA warp ================================
         // buffer = s(q)[128 x R] * U'[q][chunk rows, :]^T, A from tensor memory
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_u = umma_idesc_bf16(128, kCW);
             RingPos up;
             uint32_t n = 0;
@@ -359,7 +359,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     } else if (warp == 2) {
         // =============================== V-MMA warp ================================
         // z(q+1)[128 x R] += h_new[chunk][128 x 128] * V'[q+1][:, chunk]^T, A = the updated chunk in tensor memory
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_v = umma_idesc_bf16(128, R);
             RingPos vp;
             uint32_t n = 0;

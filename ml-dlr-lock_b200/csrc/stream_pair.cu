@@ -159,7 +159,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     volatile int* abort_flag = &bars->abort_flag;
     volatile unsigned int* stored = &bars->stored;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0);
     const int lane = threadIdx.x & 31;
     const Waiter w{abort_flag, p.spin_limit >> 2};
 
@@ -337,7 +337,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     } else if (warp == 1) {
         // =============================== U-MMA warp (leader) =======================
         // buffer = s(q)[256 x R] * U'[q][chunk rows, :]^T, A from tensor memory of both CTAs
-        if (lane == 0 && hf == 0) {
+        if (hf == 0 && elect_one()) {
             constexpr uint32_t idesc_u = umma_idesc_bf16(256, kCWP);
             RingPos up;
             uint32_t n = 0;
@@ -386,7 +386,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     } else if (warp == 2) {
         // =============================== V-MMA warp (leader) =======================
         // z(q+1)[256 x R] += h_new[chunk][256 x 128] * V'[q+1][:, chunk]^T, A = the updated chunk in tensor memory
-        if (lane == 0 && hf == 0) {
+        if (hf == 0 && elect_one()) {
             constexpr uint32_t idesc_v = umma_idesc_bf16(256, R);
             RingPos vp;
             uint32_t n = 0;
