@@ -290,7 +290,7 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di, double* esti
         std::memset(&pl, 0, sizeof(pl));
         if (dlr::stream_plan(M, d, r, L, di.num_sms, di.smem_optin, &pl) == DLRB200_OK) {
             const double t_pass = pl.cluster >= 4 ? 6.8 : (pl.cluster == 2 ? 5.5 : 2.5);
-            double t = double(pl.passes) * (L + 1) * (double(d / 128 / pl.cluster) * (r >= 256 ? 3.05 : (r >= 128 ? 1.26 : 1.15)) + t_pass);
+            double t = double(pl.passes) * (L + 1) * (double(d / 128 / pl.cluster) * (r >= 256 ? 2.25 : (r >= 128 ? 1.26 : 1.15)) + t_pass);
             if (pl.cluster == 1 && pl.grid > 100 && 4.0 * L * d * r > 100e6) t *= 1.3;
             // every layer rewrites the rows in flight in place: once they outgrow L2 (beside the weight stream)
             // each layer's traffic goes to DRAM (measured at d = 4096: 12288 / 16384 / 18944 rows in flight

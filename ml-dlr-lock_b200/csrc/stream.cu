@@ -72,8 +72,10 @@ constexpr uint32_t kZCol = 0;            // tensor-memory columns: z accumulator
 // Tensor-memory columns and shared-memory stages per rank.  Up to rank 128 there is room for two dh
 // accumulators and a separate A operand: z [0,128) | s [128,192) | A [192,256) | dh0 [256,384) | dh1 [384,512).
 // Rank 256 fills the 512 columns with z [0,256) | s [256,384) | one buffer [384,512) that holds dh and then,
-// in place, the bf16 chunk (columns 0-31 of the buffer: chunk columns 0-63, columns 64-95: chunk columns
-// 64-127); U-MMA, epilogue and V-MMA of a chunk then run one after the other.
+// in place, the bf16 chunk.  There a chunk is worked on in two halves of 64 columns, each with barriers, epilogue
+// warps and half of the buffer of its own (columns 0-63 hold dh of chunk columns 0-63, then the same as bf16 in
+// 0-31): U-MMA, epilogue and V-MMA of a half run one after the other, and the two halves fill each other's gaps.
+// d = 5120, 4096 rows: 5.45 ms with the whole chunk in one piece, 4.35 ms in halves.
 template <int R>
 struct SCfg {
     static constexpr bool ONE_BUF = R == 256;
@@ -81,14 +83,16 @@ struct SCfg {
     static constexpr uint32_t BUF_COL = ONE_BUF ? 384 : 256;
     static constexpr uint32_t A_COL = ONE_BUF ? 384 : 192;
     static constexpr int NH = ONE_BUF ? 2 : 3;           // staging slots for chunks of activations
-    // a U' stage: 128 rows x up to 128 K-columns (tiles of 64); a chunk takes USPC stages
-    static constexpr int USPC = R == 256 ? 2 : 1;
-    static constexpr int UT = R / 64 / USPC;             // tiles per stage
-    static constexpr int U_BYTES = UT * 16384;
-    // a V' stage: tiles of R rows x 64 K-columns; a chunk (128 K-columns) takes VSPC stages
-    static constexpr int VSPC = R == 256 ? 2 : 1;
+    // halves of a chunk that go through the tensor core by themselves, and a half's columns
+    static constexpr int NHALF = ONE_BUF ? 2 : 1;
+    static constexpr int HW = kCW / NHALF;
+    // a U' stage: the HW rows of a half x R K-columns, in tiles of 64
+    static constexpr int UT = R / 64;                    // tiles per stage
+    static constexpr int U_TILE_BYTES = HW * 128;
+    static constexpr int U_BYTES = UT * U_TILE_BYTES;
+    // a V' stage: R rows x the HW K-columns of a half, in tiles of 64
     static constexpr int V_TILE_BYTES = R * 128;
-    static constexpr int VT = 2 / VSPC;                  // tiles per stage
+    static constexpr int VT = HW / 64;                   // tiles per stage
     static constexpr int V_BYTES = VT * V_TILE_BYTES;
     static constexpr int NU = R == 256 ? 3 : (R == 128 ? 2 : 4);   // stages of the U' ring
     static constexpr int NV = R == 256 ? 2 : (R == 128 ? 2 : 4);   // stages of the V' ring
@@ -102,10 +106,10 @@ struct SBars {
     uint64_t h_full[kMaxNH];     // old chunk has landed (TMA bytes)
     uint64_t h_written[kMaxNH];  // the 8 epilogue warps have updated it in place
     uint64_t h_empty[kMaxNH];    // the store warp's bulk copy has read it
-    uint64_t dh_full[2];      // U-MMA warp: dh of the chunk is in the buffer
+    uint64_t dh_full[2];      // U-MMA warp: dh of the chunk is in the buffer (rank 256: per half, as the two below)
     uint64_t dh_empty[2];     // 8 epilogue warps: dh has been read
-    uint64_t a_ready;         // 8 epilogue warps: the updated chunk (bf16) is in tensor memory
-    uint64_t a_empty;         // V-MMA warp: the chunk has been read
+    uint64_t a_ready[2];      // the epilogue warps of the chunk (half): the updated chunk (bf16) is in tensor memory
+    uint64_t a_empty[2];      // V-MMA warp: the chunk (half) has been read
     uint64_t z_full, s_ready;
     uint64_t xchg_bar;        // sp > 1: the other CTAs of the cluster have published their partial z
     uint64_t ssq_bar;         // the 8 epilogue warps have published their halves of the sums of squares
@@ -182,9 +186,9 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&bars->dh_full[b]), 1);
             mbar_init(smem_u32(&bars->dh_empty[b]), kEpiWarps);
+            mbar_init(smem_u32(&bars->a_ready[b]), kEpiWarps / C::NHALF);
+            mbar_init(smem_u32(&bars->a_empty[b]), 1);
         }
-        mbar_init(smem_u32(&bars->a_ready), kEpiWarps);
-        mbar_init(smem_u32(&bars->a_empty), 1);
         mbar_init(smem_u32(&bars->z_full), 1);
         mbar_init(smem_u32(&bars->s_ready), kEpiWarps);
         mbar_init(smem_u32(&bars->ssq_bar), kEpiWarps);
@@ -232,14 +236,13 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             int uph[kMaxW], vph[kMaxW], hph[kMaxNH];   // parity of the last copy requested into each stage, -1: none
             for (int i = 0; i < kMaxW; ++i) uph[i] = vph[i] = -1;
             for (int i = 0; i < kMaxNH; ++i) hph[i] = -1;
-            const long long total_u = (long long)my_tiles * p.L * nch * C::USPC;   // stages of each weight stream
-            const long long total_v = (long long)my_tiles * p.L * nch * C::VSPC;
+            const long long total_w = (long long)my_tiles * p.L * nch * C::NHALF;   // stages of each weight stream
             const long long total_h = (long long)my_tiles * (p.L + 1) * nch;  // chunks of activations
             long long nu = 0, nv = 0, nh = 0;
             int uq = 0, uc = 0, vq = 0, vc = 0, us = 0, vs = 0;   // layer, chunk, stage within the chunk
             int ht = 0, hq = -1, hc = 0;
             uint32_t idle = 0;
-            while ((nu < total_u || nv < total_v || nh < total_h) && !err) {
+            while ((nu < total_w || nv < total_w || nh < total_h) && !err) {
                 bool did = false;
                 // pass >= 1 reads what this CTA stored one pass (nch chunks) earlier
                 if (nh < total_h && (hq < 1 || *stored + unsigned(nch) > unsigned(nh)) &&
@@ -258,20 +261,20 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     if (++hc == nch) { hc = 0; if (++hq == p.L) { hq = -1; ++ht; } }
                     did = true;
                 }
-                if (nu < total_u && mbar_test_wait(smem_u32(&bars->u_empty[up.st]), up.ph ^ 1u)) {
+                if (nu < total_w && mbar_test_wait(smem_u32(&bars->u_empty[up.st]), up.ph ^ 1u)) {
                     const uint32_t bar = smem_u32(&bars->u_full[up.st]);
                     const uint32_t dst = ubuf_s + up.st * C::U_BYTES;
                     mbar_arrive_expect_tx(bar, C::U_BYTES);
 #pragma unroll
                     for (int t = 0; t < C::UT; ++t)
-                        tma_load_2d(dst + t * 16384, &tmU, 64 * (us * C::UT + t), uq * p.d + col0 + uc * kCW, bar);
+                        tma_load_2d(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCW + us * C::HW, bar);
                     uph[up.st] = int(up.ph);
                     up.step(NU);
                     ++nu;
-                    if (++us == C::USPC) { us = 0; if (++uc == nch) { uc = 0; if (++uq == p.L) uq = 0; } }
+                    if (++us == C::NHALF) { us = 0; if (++uc == nch) { uc = 0; if (++uq == p.L) uq = 0; } }
                     did = true;
                 }
-                if (nv < total_v && mbar_test_wait(smem_u32(&bars->v_empty[vp.st]), vp.ph ^ 1u)) {
+                if (nv < total_w && mbar_test_wait(smem_u32(&bars->v_empty[vp.st]), vp.ph ^ 1u)) {
                     const uint32_t bar = smem_u32(&bars->v_full[vp.st]);
                     const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
                     mbar_arrive_expect_tx(bar, C::V_BYTES);
@@ -281,7 +284,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     vph[vp.st] = int(vp.ph);
                     vp.step(NV);
                     ++nv;
-                    if (++vs == C::VSPC) { vs = 0; if (++vc == nch) { vc = 0; if (++vq == p.L) vq = 0; } }
+                    if (++vs == C::NHALF) { vs = 0; if (++vc == nch) { vc = 0; if (++vq == p.L) vq = 0; } }
                     did = true;
                 }
                 if (did) {
@@ -305,7 +308,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         // =============================== U-MMA warp ================================
         // buffer = s(q)[128 x R] * U'[q][chunk rows, :]^T, A from tensor memory
         if (elect_one()) {
-            constexpr uint32_t idesc_u = umma_idesc_bf16(128, kCW);
+            constexpr uint32_t idesc_u = umma_idesc_bf16(128, C::HW);
             RingPos up;
             uint32_t n = 0;
             uint32_t c_s = 0;
@@ -320,35 +323,35 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     tc_fence_after();
                     mw[0] += DLS_CLK() - t0;
                     for (int c = 0; c < nch; ++c, ++n) {
-                        const uint32_t b = C::ONE_BUF ? 0u : (n & 1u);
-                        t0 = DLS_CLK();
-                        // the accumulator is free: two of them, released by the epilogue once dh is read, or the one
-                        // buffer, released by the V-MMA warp once the chunk before has been read as its A operand
-                        if (C::ONE_BUF) {
-                            if (!w.cta(smem_u32(&bars->a_empty), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
-                        } else {
-                            if (!w.cta(smem_u32(&bars->dh_empty[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
-                        }
-                        mw[2] += DLS_CLK() - t0;
-                        const uint32_t acc = tmem_base + kBufCol + b * 128u;
 #pragma unroll
-                        for (int su = 0; su < C::USPC; ++su) {
+                        for (int half = 0; half < C::NHALF; ++half) {
+                            const uint32_t b = C::ONE_BUF ? uint32_t(half) : (n & 1u);
+                            // the weights land early: wait for them first, off the critical path
                             t0 = DLS_CLK();
                             if (!w.cta(smem_u32(&bars->u_full[up.st]), up.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                             mw[1] += DLS_CLK() - t0;
+                            t0 = DLS_CLK();
+                            // the accumulator is free: two of them, released by the epilogue once dh is read, or the half
+                            // of the one buffer, released by the V-MMA warp once the chunk before has been read from it
+                            if (C::ONE_BUF) {
+                                if (!w.cta(smem_u32(&bars->a_empty[half]), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                            } else {
+                                if (!w.cta(smem_u32(&bars->dh_empty[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                            }
+                            mw[2] += DLS_CLK() - t0;
                             tc_fence_after();
+                            const uint32_t acc = tmem_base + kBufCol + b * uint32_t(C::HW);
                             const uint32_t ub = ubuf_s + up.st * C::U_BYTES;
-                            constexpr int KS = R / 16 / C::USPC;      // K steps per stage
 #pragma unroll
-                            for (int k = 0; k < KS; ++k) {
-                                const uint64_t bdesc = umma_desc(ub + uint32_t(k / 4) * 16384u, 2u, 1024u) + uint64_t(2 * (k % 4));
-                                umma_ts(acc, tmem_base + kSCol + uint32_t(8 * (su * KS + k)), bdesc, idesc_u, (su | k) ? 1u : 0u);
+                            for (int k = 0; k < R / 16; ++k) {
+                                const uint64_t bdesc = umma_desc(ub + uint32_t(k / 4) * C::U_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
+                                umma_ts(acc, tmem_base + kSCol + uint32_t(8 * k), bdesc, idesc_u, k ? 1u : 0u);
                             }
                             umma_commit(smem_u32(&bars->u_empty[up.st]));
                             up.step(NU);
+                            umma_commit(smem_u32(&bars->dh_full[b]));
                         }
                         if (err) break;
-                        umma_commit(smem_u32(&bars->dh_full[b]));
                     }
                 }
             }
@@ -369,36 +372,32 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     err_layer = q;
                     const bool feeds = q + 1 < p.L;
                     for (int c = 0; c < nch; ++c, ++n) {
-                        long long t0 = DLS_CLK();
-                        if (!w.cta(smem_u32(&bars->a_ready), n & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
-                        mw[0] += DLS_CLK() - t0;
-                        if (feeds) {
-                            const uint32_t a0 = tmem_base + kACol;
 #pragma unroll
-                            for (int sv = 0; sv < C::VSPC; ++sv) {
-                                t0 = DLS_CLK();
-                                if (!w.cta(smem_u32(&bars->v_full[vp.st]), vp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
-                                mw[1] += DLS_CLK() - t0;
+                        for (int half = 0; half < C::NHALF; ++half) {
+                            long long t0 = DLS_CLK();
+                            // the weights land early: wait for them first, off the critical path
+                            if (feeds && !w.cta(smem_u32(&bars->v_full[vp.st]), vp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                            mw[1] += DLS_CLK() - t0;
+                            t0 = DLS_CLK();
+                            if (!w.cta(smem_u32(&bars->a_ready[half]), n & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                            mw[0] += DLS_CLK() - t0;
+                            if (feeds) {
                                 tc_fence_after();
+                                const uint32_t a0 = tmem_base + kACol + uint32_t(64 * half);
                                 const uint32_t vb = vbuf_s + vp.st * C::V_BYTES;
-                                constexpr int KS = kCW / 16 / C::VSPC;    // K steps per stage
 #pragma unroll
-                                for (int kk = 0; kk < KS; ++kk) {
-                                    const int k = sv * KS + kk;          // K step of the chunk: 16 columns
-                                    const uint64_t bdesc = umma_desc(vb + uint32_t(kk / 4) * C::V_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (kk % 4));
-                                    // the chunk as A operand: 8 columns per K step, contiguous, or in two runs of
-                                    // 32 columns where it shares the buffer with dh
-                                    const uint32_t acol = C::ONE_BUF ? uint32_t(64 * (k / 4) + 8 * (k % 4)) : uint32_t(8 * k);
-                                    umma_ts(tmem_base + kZCol, a0 + acol, bdesc, idesc_v, (c | k) ? 1u : 0u);
+                                for (int k = 0; k < C::HW / 16; ++k) {     // K steps: 16 columns, 8 columns of tensor memory
+                                    const uint64_t bdesc = umma_desc(vb + uint32_t(k / 4) * C::V_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
+                                    umma_ts(tmem_base + kZCol, a0 + uint32_t(8 * k), bdesc, idesc_v, (c | half | k) ? 1u : 0u);
                                 }
                                 umma_commit(smem_u32(&bars->v_empty[vp.st]));
                                 vp.step(NV);
+                                umma_commit(smem_u32(&bars->a_empty[half]));
+                            } else {
+                                mbar_arrive(smem_u32(&bars->a_empty[half]));   // last layer: nothing reads the chunk here
                             }
-                            if (err) break;
-                            umma_commit(smem_u32(&bars->a_empty));
-                        } else {
-                            mbar_arrive(smem_u32(&bars->a_empty));   // last layer: nothing reads the chunk here
                         }
+                        if (err) break;
                     }
                     if (err) break;
                     if (feeds) umma_commit(smem_u32(&bars->z_full));
@@ -462,8 +461,10 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             for (int q = -1; q < p.L && !err; ++q) {
                 err_layer = q;
                 for (int c = 0; c < nch; ++c, ++n) {
-                    const uint32_t b = C::ONE_BUF ? 0u : (nu & 1u);
-                    const uint32_t buf = tl + kBufCol + b * 128u + uint32_t(64 * hh);
+                    // this thread's accumulator columns, and the barriers of its half
+                    const uint32_t b = C::ONE_BUF ? uint32_t(hh) : (nu & 1u);
+                    const uint32_t ab = C::ONE_BUF ? uint32_t(hh) : 0u;
+                    const uint32_t buf = tl + kBufCol + (C::ONE_BUF ? 0u : b * 128u) + uint32_t(64 * hh);
                     // ---- old values of the chunk: this thread's 128 bytes of its row, from the staging slot
                     long long t0 = DLS_CLK();
                     if (!w.cta(smem_u32(&bars->h_full[hp.st]), hp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
@@ -517,21 +518,25 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                         }
                     }
                     // ---- new values back into the staging slot, in place: the store warp copies the slot out
-                    const long long t3 = DLS_CLK();
-                    if (q >= 0) {
-                        uint8_t* rowp = hbuf + hp.st * kHBytes + hh * 16384 + er * 128;
+                    auto to_slot = [&]() {
+                        const long long t3 = DLS_CLK();
+                        if (q >= 0) {
+                            uint8_t* rowp = hbuf + hp.st * kHBytes + hh * 16384 + er * 128;
 #pragma unroll
-                        for (int ch = 0; ch < 8; ++ch)
-                            *reinterpret_cast<uint4*>(rowp + ((uint32_t(ch) ^ x7) << 4)) =
-                                make_uint4(out[4 * ch], out[4 * ch + 1], out[4 * ch + 2], out[4 * ch + 3]);
-                        fence_async_smem();
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&bars->h_written[hp.st]));
-                    ew[7] += DLS_CLK() - t3;
+                            for (int ch = 0; ch < 8; ++ch)
+                                *reinterpret_cast<uint4*>(rowp + ((uint32_t(ch) ^ x7) << 4)) =
+                                    make_uint4(out[4 * ch], out[4 * ch + 1], out[4 * ch + 2], out[4 * ch + 3]);
+                            fence_async_smem();
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&bars->h_written[hp.st]));
+                        ew[7] += DLS_CLK() - t3;
+                    };
+                    if (!C::ONE_BUF) to_slot();
                     // ---- the chunk (bf16) becomes the A operand of the next layer's contraction
                     const long long t2 = DLS_CLK();
-                    if (!w.cta(smem_u32(&bars->a_empty), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    // (rank 256: where dh came in, the buffer was free)
+                    if (!(C::ONE_BUF && q >= 0) && !w.cta(smem_u32(&bars->a_empty[ab]), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     ew[5] += DLS_CLK() - t2;
                     tc_fence_after();
                     constexpr uint32_t a_half = C::ONE_BUF ? 64u : 32u;   // in the shared buffer each thread writes over its own dh columns
@@ -540,7 +545,8 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&bars->a_ready));
+                    if (lane == 0) mbar_arrive(smem_u32(&bars->a_ready[ab]));
+                    if (C::ONE_BUF) to_slot();           // (after the hand-over that the tensor core waits for)
                     hp.step(kNH);
                     ew[6] += DLS_CLK() - t2;
                 }
@@ -730,7 +736,7 @@ int launch_stream(void* enc, const void* x, void* y, const void* Vp, const void*
     if (!encode_2d_bf16(enc, &tmX, x, uint64_t(d), uint64_t(M), 64, kRowsS, 128) ||
         !encode_2d_bf16(enc, &tmY, y, uint64_t(d), uint64_t(M), 64, kRowsS, 128) ||
         !encode_2d_bf16(enc, &tmV, Vp, uint64_t(d), uint64_t(L) * R, 64, R, 128) ||
-        !encode_2d_bf16(enc, &tmU, Up, uint64_t(R), uint64_t(L) * d, 64, 128, 128))
+        !encode_2d_bf16(enc, &tmU, Up, uint64_t(R), uint64_t(L) * d, 64, C::HW, 128))
         return DLRB200_ERR_CUDA;
     SParams p;
     p.x = static_cast<const __nv_bfloat16*>(x);

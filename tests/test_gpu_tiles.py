@@ -1,0 +1,38 @@
+"""Tensor-core kernels where their tiles can go wrong: partial tiles, one layer, several tiles per CTA."""
+import pytest
+import torch
+
+from oracle import dlrnet_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# Activations in bf16 between layers, operands rounded to bf16: the gates of the other large-batch tests.
+TOL_MODEL, TOL_TOTAL, TOL_UPDATE = 6e-3, 1e-2, 5e-2
+
+
+def _check(d, r, L, M, path):
+    import dlr_lock_b200 as D
+    dev = torch.device("cuda:0")
+    p, x = O.seeded_case(d, r, L, M, seed=d + r + L + M, alpha=1.0, gain_jitter=0.1)
+    assert D.ops.query_call(M, d, r, L).path == path
+    Vf, Uf = D.ops.fold_weights(p.V.to(dev), p.U.to(dev), p.w.to(dev), p.alpha.to(dev))
+    buf = torch.full((M + 2, d), 7.0, device=dev, dtype=torch.bfloat16)          # rows around the output stay as they are
+    y = D.ops.forward_folded(x.to(dev), Vf, Uf, p.eps, out=buf[1:M + 1])
+    again = D.ops.forward_folded(x.to(dev), Vf, Uf, p.eps)
+    torch.cuda.synchronize()
+    D.ops.check_status()
+    assert torch.equal(y, again)
+    assert bool((buf[0] == 7.0).all()) and bool((buf[M + 1] == 7.0).all())
+    model = O.forward_folded_fp32(x, Vf.cpu(), Uf.cpu(), p.eps, round_h=True)
+    want = O.forward_fp32(x, p)
+    assert O.rel_l2(y.cpu(), model) <= TOL_MODEL
+    assert O.rel_l2(y.cpu(), want) <= TOL_TOTAL
+    assert O.rel_l2_update(y.cpu(), want, x) <= TOL_UPDATE
+
+
+# rank 256, two halves per chunk: four chunks (the fewest) and more, a split of 1, 2 and 4, several tiles per CTA
+@pytest.mark.parametrize("d,L,M", [(512, 1, 65), (512, 2, 129), (640, 3, 128), (1024, 2, 66), (2048, 3, 257), (5120, 1, 130),
+                                   (512, 2, 148 * 128 + 130)])
+def test_streamed_rank_256(d, L, M, monkeypatch):
+    monkeypatch.setenv("DLRB200_FORCE_PATH", "4")
+    _check(d, 256, L, M, 4)
