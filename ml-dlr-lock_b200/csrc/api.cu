@@ -229,17 +229,16 @@ int check_shape(int M, int d, int r, int L) {
 //                    cluster when that still fits the GPU
 // All were timed on a B200 over widths 512..8192, ranks 64 and 128 and 512..32768 rows; the choice is a cost
 // model fitted to those times (microseconds):
-//   cluster   waves * L * t_layer, t_layer = 8.2 (r = 128) or 6.4 (r = 64) whatever the width
+//   cluster   waves * L * t_layer, t_layer by rank and stripe (layer_us in cluster.cu: 3.2 to 7.5)
 //   streamed  waves * (L + 1) * (chunks per CTA * t_chunk + t_pass), t_chunk = 1.26 (r = 128) or 1.15 (r = 64),
 //             t_pass = 2.5 / 5.5 / 6.8 for a split of 1 / 2 / 4 (normalise + SiLU, and the exchange); 30 % more
 //             when over 100 unsplit CTAs stream weights that do not fit in L2
-//   pairs     waves * (L + 1) * (chunks per pair * t_chunk + t_pass), t_chunk = 1.09 (r = 128) or 0.80 (r = 64),
-//             t_pass = 4.4 with two pairs per cluster (exchange in distributed shared memory), 2.5 with one.
+//   pairs     waves * (L + 1) * (chunks per pair * t_chunk + t_pass), t_chunk = 0.98 (r = 128) or 0.85 (r = 64),
+//             t_pass = 4.6 or 2.8 with two pairs per cluster (exchange in distributed shared memory), 1.0 less with one.
 //             One pair per cluster at rank 128 means at least 9000 rows, where the activations no longer fit in
 //             L2 and the unsplit streamed kernel is as fast or faster: not taken there.
-// At d = 4096, r = 128, L = 143 (ms, cluster / streamed / pairs): 2048 rows 2.34 / 2.47 / 3.09, 4096 rows
-// 3.55 / 2.49 / 3.08, 6144 rows 4.72 / 3.66 / 3.10, 8192 rows 6.37 / 3.86 / 3.14, 16384 rows 12.1 / 7.97 / 8.71.
-// At d = 2048, r = 64, L = 142: 8192 rows 1.82 / 1.98 / 1.51, 16384 rows 3.66 / 2.97 / 2.70.
+// At d = 4096, r = 128, L = 143 (ms, cluster / pairs): 1900 rows 1.09 / 1.85, 2048 rows 2.04 / 1.85, 3840 rows 2.17 / 1.87.
+// At d = 2048, r = 64, L = 142: 4096 rows 0.76 / 1.37, 8192 rows 1.52 / 1.38.
 // Shapes the cluster kernel does not cover (d > 4096, d not a multiple of 512, r > d / 32) stream.
 struct RouteEntry {
     int tiles, d, r, L, sms, path;         // the plans depend on M only through the number of 128-row tiles
@@ -281,8 +280,9 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di, double* esti
     dlrb200_plan pl;
     if (can_cluster) {
         std::memset(&pl, 0, sizeof(pl));
-        if (dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, &pl) == DLRB200_OK) {
-            best = 0.97 * double(pl.passes) * L * (r >= 128 ? 8.2 : (r >= 64 ? 6.4 : 5.5));     // ties go to the cluster kernel
+        double us = 0.0;
+        if (dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, &pl, &us, false) == DLRB200_OK) {
+            best = 0.97 * us;                            // ties go to the cluster kernel
             path = DLRB200_PATH_CLUSTER;
         }
     }
@@ -308,8 +308,8 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di, double* esti
             const int pp = pl.cluster / 2;
             // (measured only where the pairs cover most of the GPU: not taken for smaller grids)
             if (pp == 4 || ((pp == 2 || r == 64) && pl.grid >= 96)) {
-                const double pause = (r >= 128 ? 3.4 : 2.0) + (pp == 4 ? 2.8 : (pp == 2 ? 1.0 : 0.0));
-                const double t = double(pl.passes) * (L + 1) * (double(d / 128 / pp) * (r >= 128 ? 1.09 : 0.80) + pause);
+                const double pause = (r >= 128 ? 3.6 : 1.8) + (pp == 4 ? (r >= 128 ? 1.4 : 1.9) : (pp == 2 ? 1.0 : 0.0));
+                const double t = double(pl.passes) * (L + 1) * (double(d / 128 / pp) * (r >= 128 ? 0.98 : 0.85) + pause);
                 if (t < best) { best = t; path = DLRB200_PATH_STREAMED_PAIRS; }
             }
         }
@@ -489,7 +489,7 @@ int dlrb200_query(int M, int d, int r, int L, dlrb200_plan* plan) {
         plan->workspace_bytes = ws;
         return rc;
     }
-    if (use_cluster_path(M, d, r, L)) return dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, plan);
+    if (use_cluster_path(M, d, r, L)) return dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, plan, nullptr, true);
     if (use_cluster_small(M, d, r)) return dlr::decode_cluster_plan(M, d, r, L, di.smem_optin, plan);
     const int dc = pick_stripe_cols(d, di.num_sms);
     if (dc == 0) return DLRB200_ERR_UNSUPPORTED_SHAPE;
@@ -509,6 +509,7 @@ int dlrb200_query_call(int M, int d, int r, int L, dlrb200_plan* plan) {
     if (device_info(&di) != DLRB200_OK) return DLRB200_ERR_CUDA;
     dlrb200_plan resident = *plan;
     if (use_resident(M, d, r, L, di, &resident)) *plan = resident;
+    else if (plan->path == DLRB200_PATH_CLUSTER) return dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, plan, nullptr, false);
     return DLRB200_OK;
 }
 

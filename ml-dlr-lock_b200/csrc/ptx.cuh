@@ -129,12 +129,12 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 // non-zero.  One block of assembly with uniform branches: every lane polls the same word, so the warp never splits, and
 // a look at a phase that is already complete costs about 60 cycles against 100 for the same loop in C++ (measured; the
 // difference is the bookkeeping for lanes that leave a loop at different times).  `limit` must not be 0.
-#define DLR_MBAR_WAIT_FLAG(NAME, FORM)                                                                              \
+#define DLR_MBAR_WAIT_FLAG(NAME, FORM, AGREE)                                                                       \
     __device__ __forceinline__ bool NAME(uint32_t bar, uint32_t parity, uint32_t flag, uint32_t limit) {            \
         uint32_t ok;                                                                                                \
         asm volatile(                                                                                               \
             "{\n\t.reg .pred P1, P2;\n\t.reg .u32 n, f;\n\tmov.u32 n, %4;\n"                                          \
-            "DLR_WAIT_%=:\n\t" FORM " P1, [%1], %2;\n\t@P1 bra.uni DLR_DONE_%=;\n\t"                                  \
+            "DLR_WAIT_%=:\n\t" FORM " P1, [%1], %2;\n\t" AGREE "@P1 bra.uni DLR_DONE_%=;\n\t"                            \
             "ld.volatile.shared.u32 f, [%3];\n\tsub.u32 n, n, 1;\n\tsetp.ne.u32 P2, n, 0;\n\t"                      \
             "setp.eq.and.u32 P2, f, 0, P2;\n\t@P2 bra.uni DLR_WAIT_%=;\n"                                            \
             "DLR_DONE_%=:\n\tselp.u32 %0, 1, 0, P1;\n\t}"                                                           \
@@ -143,9 +143,17 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
             : "memory");                                                                                            \
         return ok != 0;                                                                                             \
     }
-DLR_MBAR_WAIT_FLAG(mbar_wait_flag, "mbarrier.try_wait.parity.shared::cta.b64")
+DLR_MBAR_WAIT_FLAG(mbar_wait_flag, "mbarrier.try_wait.parity.shared::cta.b64", "")
 // ... acquiring at cluster scope, for arrivals and stores that come from other CTAs
-DLR_MBAR_WAIT_FLAG(mbar_wait_flag_cluster, "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64")
+DLR_MBAR_WAIT_FLAG(mbar_wait_flag_cluster, "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64", "")
+// The same for a converged warp, all of whose lanes agree on each look (and on the flag, one word read in one instruction).
+// The warps of the tensor-core kernels wait with these, the issuing warps too, which elect a lane only for the instructions
+// of a chunk: a look by one lane of a split warp costs about 250 cycles.  Measured in the cluster kernel (us, issue and
+// copy warps as one elected thread / whole): d = 1024, 4096 rows 482 / 454; d = 4096, 1000 rows 1136 / 1064.
+#define DLR_AGREE "vote.sync.all.pred P1, P1, 0xffffffff;\n\t"
+DLR_MBAR_WAIT_FLAG(mbar_wait_warp, "mbarrier.try_wait.parity.shared::cta.b64", DLR_AGREE)
+DLR_MBAR_WAIT_FLAG(mbar_wait_warp_cluster, "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64", DLR_AGREE)
+#undef DLR_AGREE
 #undef DLR_MBAR_WAIT_FLAG
 
 // Polls granted to the waits that run only when a kernel is giving up: copies and
@@ -472,7 +480,12 @@ __device__ __forceinline__ void st_async_v4(uint32_t dst_cluster, uint32_t a, ui
                  : "memory");
 }
 
-// The same for one 32-bit word.
+// The same for 8 bytes, and for one 32-bit word.
+__device__ __forceinline__ void st_async_v2(uint32_t dst_cluster, uint32_t a, uint32_t b, uint32_t bar_cluster) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(dst_cluster),
+                 "r"(a), "r"(b), "r"(bar_cluster)
+                 : "memory");
+}
 __device__ __forceinline__ void st_async_b32(uint32_t dst_cluster, uint32_t a, uint32_t bar_cluster) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst_cluster), "r"(a),
                  "r"(bar_cluster)

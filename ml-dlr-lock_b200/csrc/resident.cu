@@ -107,12 +107,6 @@ struct RBars {
 };
 static_assert(sizeof(RBars) <= 1024, "barrier block");
 
-__device__ __forceinline__ void st_async_v2(uint32_t dst_cluster, uint32_t a, uint32_t b, uint32_t bar_cluster) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(dst_cluster),
-                 "r"(a), "r"(b), "r"(bar_cluster)
-                 : "memory");
-}
-
 // 8 x 8 transposition of packed 16-bit values across a warp
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     uint32_t r;

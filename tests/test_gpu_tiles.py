@@ -36,3 +36,16 @@ def _check(d, r, L, M, path):
 def test_streamed_rank_256(d, L, M, monkeypatch):
     monkeypatch.setenv("DLRB200_FORCE_PATH", "4")
     _check(d, 256, L, M, 4)
+
+
+# the cluster kernel: both stripes, partial tiles, one layer, fewer and more tiles than clusters fit on the GPU at once
+@pytest.mark.parametrize("stripe", [512, 256])
+@pytest.mark.parametrize("d,r,L,M", [(512, 32, 3, 65), (512, 64, 2, 129), (512, 128, 1, 130), (1024, 32, 3, 257), (1024, 64, 1, 100),
+                                     (1024, 128, 2, 384), (2048, 64, 2, 333), (2048, 128, 3, 128), (4096, 128, 2, 200),
+                                     (512, 32, 2, 148 * 128 + 70), (1024, 32, 2, 74 * 128 + 1), (2048, 128, 2, 37 * 128 + 70)])
+def test_cluster_kernel(d, r, L, M, stripe, monkeypatch):
+    import dlr_lock_b200 as D
+    monkeypatch.setenv("DLRB200_FORCE_PATH", "2")
+    monkeypatch.setenv("DLRB200_CLUSTER_STRIPE", str(stripe))
+    assert D.ops.query_call(M, d, r, L).stripe_cols == (512 if d > 2048 else stripe)
+    _check(d, r, L, M, 2)
