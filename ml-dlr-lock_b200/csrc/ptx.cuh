@@ -492,38 +492,6 @@ __device__ __forceinline__ void st_async_b32(uint32_t dst_cluster, uint32_t a, u
                  : "memory");
 }
 
-// Bounded waits on mbarriers that also give up when another thread of the CTA has
-// raised the abort flag (a word in shared memory).
-struct Waiter {
-    volatile int* abort_flag;
-    uint32_t limit;
-    __device__ __forceinline__ bool cta(uint32_t bar, uint32_t parity) const {
-        for (uint32_t i = 0; i < limit; ++i) {
-            if (mbar_try_wait(bar, parity)) return true;
-            if ((i & 63u) == 63u && *abort_flag) return false;
-        }
-        return false;
-    }
-    // Whole warp, every lane with a barrier and parity of its own (lanes may name the same one): one poll
-    // covers several barriers at the latency of one.  Returns true once every lane's phase is complete.
-    __device__ __forceinline__ bool warp(uint32_t bar, uint32_t parity) const {
-        bool done = false;
-        for (uint32_t i = 0; i < limit; ++i) {
-            if (!done) done = mbar_try_wait(bar, parity);
-            if (__all_sync(0xffffffffu, done)) return true;
-            if ((i & 63u) == 63u && *abort_flag) return false;
-        }
-        return false;
-    }
-    __device__ __forceinline__ bool cluster(uint32_t bar, uint32_t parity) const {
-        for (uint32_t i = 0; i < limit; ++i) {
-            if (mbar_try_wait_cluster(bar, parity)) return true;
-            if ((i & 63u) == 63u && *abort_flag) return false;
-        }
-        return false;
-    }
-};
-
 // ---------------------------------------------------------------------------
 // TMA store (shared -> global through a tensor map) and its bulk groups
 // ---------------------------------------------------------------------------

@@ -169,7 +169,10 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0);
     const int lane = threadIdx.x & 31;
-    const Waiter w{abort_flag, p.spin_limit >> 2};
+    const uint32_t flag_s = smem_u32(&bars->abort_flag);
+    const uint32_t limit = p.spin_limit >= 4 ? p.spin_limit >> 2 : 1u;
+    auto wait_cta = [&](uint32_t bar, uint32_t parity) { return mbar_wait_warp(bar, parity, flag_s, limit); };
+    auto wait_cluster = [&](uint32_t bar, uint32_t parity) { return mbar_wait_warp_cluster(bar, parity, flag_s, limit); };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxW; ++s) {
@@ -231,11 +234,10 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     if (warp == 0) {
         // =============================== TMA producer ===============================
         // The two rings advance independently: whichever has a free stage gets its next tile.
-        if (lane == 0) {
+        // (the whole warp looks at the barriers, one lane issues: see mbar_wait_warp)
+        {
             RingPos up, vp, hp;
-            int uph[kMaxW], vph[kMaxW], hph[kMaxNH];   // parity of the last copy requested into each stage, -1: none
-            for (int i = 0; i < kMaxW; ++i) uph[i] = vph[i] = -1;
-            for (int i = 0; i < kMaxNH; ++i) hph[i] = -1;
+            auto free_stage = [&](bool want, uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, want && mbar_test_wait(smem_u32(bar), parity)) != 0; };
             const long long total_w = (long long)my_tiles * p.L * nch * C::NHALF;   // stages of each weight stream
             const long long total_h = (long long)my_tiles * (p.L + 1) * nch;  // chunks of activations
             long long nu = 0, nv = 0, nh = 0;
@@ -245,43 +247,48 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             while ((nu < total_w || nv < total_w || nh < total_h) && !err) {
                 bool did = false;
                 // pass >= 1 reads what this CTA stored one pass (nch chunks) earlier
-                if (nh < total_h && (hq < 1 || *stored + unsigned(nch) > unsigned(nh)) &&
-                    mbar_test_wait(smem_u32(&bars->h_empty[hp.st]), hp.ph ^ 1u)) {
-                    if (hq >= 1) asm volatile("fence.proxy.async.global;" ::: "memory");
-                    const uint32_t bar = smem_u32(&bars->h_full[hp.st]);
-                    const uint32_t dst = hbuf_s + hp.st * kHBytes;
-                    const CUtensorMap* src = hq >= 1 ? &tmY : &tmX;
-                    const int m0 = (cl + ht * ncl) * kRowsS;
-                    mbar_arrive_expect_tx(bar, kHBytes);
-                    tma_load_2d(dst, src, col0 + hc * kCW, m0, bar);
-                    tma_load_2d(dst + 16384, src, col0 + hc * kCW + 64, m0, bar);
-                    hph[hp.st] = int(hp.ph);
+                if (free_stage(nh < total_h && (hq < 1 || *stored + unsigned(nch) > unsigned(nh)), &bars->h_empty[hp.st], hp.ph ^ 1u)) {
+                    if (elect_one()) {
+                        if (hq >= 1) asm volatile("fence.proxy.async.global;" ::: "memory");
+                        const uint32_t bar = smem_u32(&bars->h_full[hp.st]);
+                        const uint32_t dst = hbuf_s + hp.st * kHBytes;
+                        const CUtensorMap* src = hq >= 1 ? &tmY : &tmX;
+                        const int m0 = (cl + ht * ncl) * kRowsS;
+                        mbar_arrive_expect_tx(bar, kHBytes);
+                        tma_load_2d(dst, src, col0 + hc * kCW, m0, bar);
+                        tma_load_2d(dst + 16384, src, col0 + hc * kCW + 64, m0, bar);
+                    }
+                    __syncwarp();
                     hp.step(kNH);
                     ++nh;
                     if (++hc == nch) { hc = 0; if (++hq == p.L) { hq = -1; ++ht; } }
                     did = true;
                 }
-                if (nu < total_w && mbar_test_wait(smem_u32(&bars->u_empty[up.st]), up.ph ^ 1u)) {
-                    const uint32_t bar = smem_u32(&bars->u_full[up.st]);
-                    const uint32_t dst = ubuf_s + up.st * C::U_BYTES;
-                    mbar_arrive_expect_tx(bar, C::U_BYTES);
+                if (free_stage(nu < total_w, &bars->u_empty[up.st], up.ph ^ 1u)) {
+                    if (elect_one()) {
+                        const uint32_t bar = smem_u32(&bars->u_full[up.st]);
+                        const uint32_t dst = ubuf_s + up.st * C::U_BYTES;
+                        mbar_arrive_expect_tx(bar, C::U_BYTES);
 #pragma unroll
-                    for (int t = 0; t < C::UT; ++t)
-                        tma_load_2d(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCW + us * C::HW, bar);
-                    uph[up.st] = int(up.ph);
+                        for (int t = 0; t < C::UT; ++t)
+                            tma_load_2d(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCW + us * C::HW, bar);
+                    }
+                    __syncwarp();
                     up.step(NU);
                     ++nu;
                     if (++us == C::NHALF) { us = 0; if (++uc == nch) { uc = 0; if (++uq == p.L) uq = 0; } }
                     did = true;
                 }
-                if (nv < total_w && mbar_test_wait(smem_u32(&bars->v_empty[vp.st]), vp.ph ^ 1u)) {
-                    const uint32_t bar = smem_u32(&bars->v_full[vp.st]);
-                    const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
-                    mbar_arrive_expect_tx(bar, C::V_BYTES);
+                if (free_stage(nv < total_w, &bars->v_empty[vp.st], vp.ph ^ 1u)) {
+                    if (elect_one()) {
+                        const uint32_t bar = smem_u32(&bars->v_full[vp.st]);
+                        const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
+                        mbar_arrive_expect_tx(bar, C::V_BYTES);
 #pragma unroll
-                    for (int t = 0; t < C::VT; ++t)
-                        tma_load_2d(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCW + 64 * (vs * C::VT + t), vq * R, bar);
-                    vph[vp.st] = int(vp.ph);
+                        for (int t = 0; t < C::VT; ++t)
+                            tma_load_2d(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCW + 64 * (vs * C::VT + t), vq * R, bar);
+                    }
+                    __syncwarp();
                     vp.step(NV);
                     ++nv;
                     if (++vs == C::NHALF) { vs = 0; if (++vc == nch) { vc = 0; if (++vq == p.L) vq = 0; } }
@@ -289,25 +296,25 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 }
                 if (did) {
                     idle = 0;
-                } else if (++idle > p.spin_limit || ((idle & 63u) == 63u && *abort_flag)) {
+                } else if (++idle, __any_sync(0xffffffffu, idle > p.spin_limit || ((idle & 63u) == 63u && *abort_flag))) {
                     err = DLRB200_ERR_TIMEOUT_COPY;
                     err_layer = uq;
                 }
             }
             if (err || *abort_flag) {
                 // copies requested before giving up still land in this CTA's shared memory: wait for them
-                for (int i = 0; i < int(kNH); ++i)
-                    if (hph[i] >= 0) mbar_wait(smem_u32(&bars->h_full[i]), uint32_t(hph[i]), kDrainPolls);
-                for (int i = 0; i < int(NU); ++i)
-                    if (uph[i] >= 0) mbar_wait(smem_u32(&bars->u_full[i]), uint32_t(uph[i]), kDrainPolls);
-                for (int i = 0; i < int(NV); ++i)
-                    if (vph[i] >= 0) mbar_wait(smem_u32(&bars->v_full[i]), uint32_t(vph[i]), kDrainPolls);
+                for (long long m = nh - 1; m >= 0 && m >= nh - int(kNH); --m)
+                    mbar_wait(smem_u32(&bars->h_full[m % kNH]), uint32_t(m / kNH) & 1u, kDrainPolls);
+                for (long long m = nu - 1; m >= 0 && m >= nu - int(NU); --m)
+                    mbar_wait(smem_u32(&bars->u_full[m % NU]), uint32_t(m / NU) & 1u, kDrainPolls);
+                for (long long m = nv - 1; m >= 0 && m >= nv - int(NV); --m)
+                    mbar_wait(smem_u32(&bars->v_full[m % NV]), uint32_t(m / NV) & 1u, kDrainPolls);
             }
         }
     } else if (warp == 1) {
         // =============================== U-MMA warp ================================
         // buffer = s(q)[128 x R] * U'[q][chunk rows, :]^T, A from tensor memory
-        if (elect_one()) {
+        {
             constexpr uint32_t idesc_u = umma_idesc_bf16(128, C::HW);
             RingPos up;
             uint32_t n = 0;
@@ -318,7 +325,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 for (int q = 0; q < p.L && !err; ++q) {
                     err_layer = q;
                     long long t0 = DLS_CLK();
-                    if (!w.cta(smem_u32(&bars->s_ready), c_s & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cta(smem_u32(&bars->s_ready), c_s & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     ++c_s;
                     tc_fence_after();
                     mw[0] += DLS_CLK() - t0;
@@ -328,41 +335,45 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                             const uint32_t b = C::ONE_BUF ? uint32_t(half) : (n & 1u);
                             // the weights land early: wait for them first, off the critical path
                             t0 = DLS_CLK();
-                            if (!w.cta(smem_u32(&bars->u_full[up.st]), up.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                            if (!wait_cta(smem_u32(&bars->u_full[up.st]), up.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                             mw[1] += DLS_CLK() - t0;
                             t0 = DLS_CLK();
                             // the accumulator is free: two of them, released by the epilogue once dh is read, or the half
                             // of the one buffer, released by the V-MMA warp once the chunk before has been read from it
                             if (C::ONE_BUF) {
-                                if (!w.cta(smem_u32(&bars->a_empty[half]), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                                if (!wait_cta(smem_u32(&bars->a_empty[half]), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                             } else {
-                                if (!w.cta(smem_u32(&bars->dh_empty[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                                if (!wait_cta(smem_u32(&bars->dh_empty[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                             }
                             mw[2] += DLS_CLK() - t0;
                             tc_fence_after();
                             const uint32_t acc = tmem_base + kBufCol + b * uint32_t(C::HW);
                             const uint32_t ub = ubuf_s + up.st * C::U_BYTES;
+                            if (elect_one()) {
 #pragma unroll
-                            for (int k = 0; k < R / 16; ++k) {
-                                const uint64_t bdesc = umma_desc(ub + uint32_t(k / 4) * C::U_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
-                                umma_ts(acc, tmem_base + kSCol + uint32_t(8 * k), bdesc, idesc_u, k ? 1u : 0u);
+                                for (int k = 0; k < R / 16; ++k) {
+                                    const uint64_t bdesc = umma_desc(ub + uint32_t(k / 4) * C::U_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
+                                    umma_ts(acc, tmem_base + kSCol + uint32_t(8 * k), bdesc, idesc_u, k ? 1u : 0u);
+                                }
+                                umma_commit(smem_u32(&bars->u_empty[up.st]));
+                                umma_commit(smem_u32(&bars->dh_full[b]));
                             }
-                            umma_commit(smem_u32(&bars->u_empty[up.st]));
+                            __syncwarp();
                             up.step(NU);
-                            umma_commit(smem_u32(&bars->dh_full[b]));
                         }
                         if (err) break;
                     }
                 }
             }
-            umma_commit(smem_u32(&bars->drain[0]));
+            if (elect_one()) umma_commit(smem_u32(&bars->drain[0]));
+            __syncwarp();
             mbar_wait(smem_u32(&bars->drain[0]), 0, kDrainPolls);
-            if (p.prof) for (int k = 0; k < 3; ++k) p.prof[blockIdx.x * 32 + 4 + k] = (unsigned long long)mw[k];
+            if (p.prof && lane == 0) for (int k = 0; k < 3; ++k) p.prof[blockIdx.x * 32 + 4 + k] = (unsigned long long)mw[k];
         }
     } else if (warp == 2) {
         // =============================== V-MMA warp ================================
         // z(q+1)[128 x R] += h_new[chunk][128 x 128] * V'[q+1][:, chunk]^T, A = the updated chunk in tensor memory
-        if (elect_one()) {
+        {
             constexpr uint32_t idesc_v = umma_idesc_bf16(128, R);
             RingPos vp;
             uint32_t n = 0;
@@ -376,43 +387,48 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                         for (int half = 0; half < C::NHALF; ++half) {
                             long long t0 = DLS_CLK();
                             // the weights land early: wait for them first, off the critical path
-                            if (feeds && !w.cta(smem_u32(&bars->v_full[vp.st]), vp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                            if (feeds && !wait_cta(smem_u32(&bars->v_full[vp.st]), vp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                             mw[1] += DLS_CLK() - t0;
                             t0 = DLS_CLK();
-                            if (!w.cta(smem_u32(&bars->a_ready[half]), n & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                            if (!wait_cta(smem_u32(&bars->a_ready[half]), n & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                             mw[0] += DLS_CLK() - t0;
                             if (feeds) {
                                 tc_fence_after();
                                 const uint32_t a0 = tmem_base + kACol + uint32_t(64 * half);
                                 const uint32_t vb = vbuf_s + vp.st * C::V_BYTES;
+                                if (elect_one()) {
 #pragma unroll
-                                for (int k = 0; k < C::HW / 16; ++k) {     // K steps: 16 columns, 8 columns of tensor memory
-                                    const uint64_t bdesc = umma_desc(vb + uint32_t(k / 4) * C::V_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
-                                    umma_ts(tmem_base + kZCol, a0 + uint32_t(8 * k), bdesc, idesc_v, (c | half | k) ? 1u : 0u);
+                                    for (int k = 0; k < C::HW / 16; ++k) {     // K steps: 16 columns, 8 columns of tensor memory
+                                        const uint64_t bdesc = umma_desc(vb + uint32_t(k / 4) * C::V_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
+                                        umma_ts(tmem_base + kZCol, a0 + uint32_t(8 * k), bdesc, idesc_v, (c | half | k) ? 1u : 0u);
+                                    }
+                                    umma_commit(smem_u32(&bars->v_empty[vp.st]));
+                                    umma_commit(smem_u32(&bars->a_empty[half]));
                                 }
-                                umma_commit(smem_u32(&bars->v_empty[vp.st]));
+                                __syncwarp();
                                 vp.step(NV);
-                                umma_commit(smem_u32(&bars->a_empty[half]));
                             } else {
-                                mbar_arrive(smem_u32(&bars->a_empty[half]));   // last layer: nothing reads the chunk here
+                                if (lane == 0) mbar_arrive(smem_u32(&bars->a_empty[half]));   // last layer: nothing reads the chunk here
                             }
                         }
                         if (err) break;
                     }
                     if (err) break;
-                    if (feeds) umma_commit(smem_u32(&bars->z_full));
+                    if (feeds && elect_one()) umma_commit(smem_u32(&bars->z_full));
+                    __syncwarp();
                 }
             }
-            umma_commit(smem_u32(&bars->drain[1]));
+            if (elect_one()) umma_commit(smem_u32(&bars->drain[1]));
+            __syncwarp();
             mbar_wait(smem_u32(&bars->drain[1]), 0, kDrainPolls);
-            if (p.prof) for (int k = 0; k < 2; ++k) p.prof[blockIdx.x * 32 + 8 + k] = (unsigned long long)mw[k];
+            if (p.prof && lane == 0) for (int k = 0; k < 2; ++k) p.prof[blockIdx.x * 32 + 8 + k] = (unsigned long long)mw[k];
         }
     } else if (warp == 3) {
         // =============================== store warp ================================
         // updated chunk -> output buffer.  The slot is released when the copy has read it; the chunk counts as
         // stored (readable by the next pass) once its bulk group is complete, which is checked two chunks late
         // so that this warp never waits for a write in flight.
-        if (lane == 0) {
+        {
             RingPos hp;
             unsigned int n = 0;              // chunks seen (all tiles, all passes): the producer counts the same way
             for (int t = 0; t < my_tiles && !err; ++t) {
@@ -420,26 +436,29 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 for (int q = -1; q < p.L && !err; ++q) {
                     err_layer = q;
                     for (int c = 0; c < nch; ++c, ++n) {
-                        if (!w.cta(smem_u32(&bars->h_written[hp.st]), hp.ph)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
-                        if (q >= 0) {
-                            const uint32_t src = hbuf_s + hp.st * kHBytes;
-                            tma_store_2d(&tmY, col0 + c * kCW, m0, src);
-                            tma_store_2d(&tmY, col0 + c * kCW + 64, m0, src + 16384);
-                            bulk_commit_group();
-                            bulk_wait_group_read<0>();
-                            bulk_wait_group<2>();            // every group but the last two is complete
-                            if (n + 1u > *stored + 2u) *stored = n + 1u - 2u;
-                        } else {
-                            // the pass over x stores nothing; also the point where the tile before is fully stored
-                            bulk_wait_group<0>();
-                            *stored = n + 1u;
+                        if (!wait_cta(smem_u32(&bars->h_written[hp.st]), hp.ph)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (lane == 0) {           // (bulk groups belong to a thread)
+                            if (q >= 0) {
+                                const uint32_t src = hbuf_s + hp.st * kHBytes;
+                                tma_store_2d(&tmY, col0 + c * kCW, m0, src);
+                                tma_store_2d(&tmY, col0 + c * kCW + 64, m0, src + 16384);
+                                bulk_commit_group();
+                                bulk_wait_group_read<0>();
+                                bulk_wait_group<2>();            // every group but the last two is complete
+                                if (n + 1u > *stored + 2u) *stored = n + 1u - 2u;
+                            } else {
+                                // the pass over x stores nothing; also the point where the tile before is fully stored
+                                bulk_wait_group<0>();
+                                *stored = n + 1u;
+                            }
+                            mbar_arrive(smem_u32(&bars->h_empty[hp.st]));
                         }
-                        mbar_arrive(smem_u32(&bars->h_empty[hp.st]));
+                        __syncwarp();
                         hp.step(kNH);
                     }
                 }
             }
-            bulk_wait_group<0>();
+            if (lane == 0) bulk_wait_group<0>();
         }
     } else if (warp >= 4) {
         // =============================== epilogue warps =============================
@@ -467,7 +486,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     const uint32_t buf = tl + kBufCol + (C::ONE_BUF ? 0u : b * 128u) + uint32_t(64 * hh);
                     // ---- old values of the chunk: this thread's 128 bytes of its row, from the staging slot
                     long long t0 = DLS_CLK();
-                    if (!w.cta(smem_u32(&bars->h_full[hp.st]), hp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                    if (!wait_cta(smem_u32(&bars->h_full[hp.st]), hp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                     ew[4] += DLS_CLK() - t0;
                     uint32_t cur[32];
                     {
@@ -481,7 +500,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     uint32_t out[32];
                     t0 = DLS_CLK();
                     if (q >= 0) {
-                        if (!w.cta(smem_u32(&bars->dh_full[b]), (C::ONE_BUF ? nu : (nu >> 1)) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (!wait_cta(smem_u32(&bars->dh_full[b]), (C::ONE_BUF ? nu : (nu >> 1)) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         ++nu;
                         ew[1] += DLS_CLK() - t0;
                         tc_fence_after();
@@ -536,7 +555,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     // ---- the chunk (bf16) becomes the A operand of the next layer's contraction
                     const long long t2 = DLS_CLK();
                     // (rank 256: where dh came in, the buffer was free)
-                    if (!(C::ONE_BUF && q >= 0) && !w.cta(smem_u32(&bars->a_empty[ab]), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!(C::ONE_BUF && q >= 0) && !wait_cta(smem_u32(&bars->a_empty[ab]), (n & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     ew[5] += DLS_CLK() - t2;
                     tc_fence_after();
                     constexpr uint32_t a_half = C::ONE_BUF ? 64u : 32u;   // in the shared buffer each thread writes over its own dh columns
@@ -556,7 +575,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     const long long t0 = DLS_CLK();
                     constexpr int NZ = R / 2;            // columns of z per thread, handled 32 at a time
                     constexpr int NQ = NZ / 8 + 1;       // 16-byte words a thread publishes: z as bf16 pairs, then its sum of squares
-                    if (!w.cta(smem_u32(&bars->z_full), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cta(smem_u32(&bars->z_full), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     tc_fence_after();
                     const long long tb1 = DLS_CLK();
                     ew[8] += tb1 - t0;
@@ -588,7 +607,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                                 mbar_arrive_remote(mapa(smem_u32(&bars->xchg_bar), uint32_t((rank + o) % sp)));
                         const long long tb2 = DLS_CLK();
                         ew[9] += tb2 - tb1;
-                        if (!w.cluster(smem_u32(&bars->xchg_bar), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (!wait_cluster(smem_u32(&bars->xchg_bar), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         ew[10] += DLS_CLK() - tb2;
                         float qs = 0.f;
                         for (int o = 0; o < sp; ++o)
@@ -599,7 +618,7 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     ssqx[hh * kRowsS + er] = ssq;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bars->ssq_bar));
-                    if (!w.cta(smem_u32(&bars->ssq_bar), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cta(smem_u32(&bars->ssq_bar), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     ew[11] += DLS_CLK() - tb3;
                     const float tot = ssq + ssqx[(hh ^ 1) * kRowsS + er];
                     const float rstd = rsqrtf(tot * p.inv_d + p.eps);

@@ -38,6 +38,10 @@
 // barrier: no fences, no trip through global memory), and both sides add own
 // (rounded alike) + received: every CTA ends with the same bits.
 //
+// Every role waits as a whole warp and elects a lane for what one thread does (a
+// look at a barrier by one lane of a split warp costs about 250 cycles): d = 4096,
+// 8192 rows, back to back: 3.27 ms with one thread per role, 2.97 ms so.
+//
 // All waits are bounded; a wait that gives up raises an abort flag, records a
 // status word and every role drains and leaves.
 #include <cstdlib>
@@ -161,7 +165,10 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0);
     const int lane = threadIdx.x & 31;
-    const Waiter w{abort_flag, p.spin_limit >> 2};
+    const uint32_t flag_s = smem_u32(&bars->abort_flag);
+    const uint32_t limit = p.spin_limit >= 4 ? p.spin_limit >> 2 : 1u;
+    auto wait_cta = [&](uint32_t bar, uint32_t parity) { return mbar_wait_warp(bar, parity, flag_s, limit); };
+    auto wait_cluster = [&](uint32_t bar, uint32_t parity) { return mbar_wait_warp_cluster(bar, parity, flag_s, limit); };
 
     const int pp = p.pp;
     const uint32_t crank = cluster_ctarank();
@@ -232,11 +239,10 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     // feeds the V contraction of layer q+1.  Chunk number n (all tiles, all passes) uses buffer n & 1.
     if (warp == 0) {
         // =============================== TMA producer ===============================
-        if (lane == 0) {
+        // (the whole warp looks at the barriers, one lane issues: see mbar_wait_warp)
+        {
             RingPos up, vp, hp;
-            int uph[kMaxWP], vph[kMaxWP], hph[kNLP];   // parity of the last copy requested into each stage, -1: none
-            for (int i = 0; i < kMaxWP; ++i) uph[i] = vph[i] = -1;
-            for (int i = 0; i < kNLP; ++i) hph[i] = -1;
+            auto free_stage = [&](bool want, uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, want && mbar_test(smem_u32(bar), parity)) != 0; };
             const long long total_w = (long long)my_tiles * p.L * nch;        // stages of each weight stream
             const long long total_h = (long long)my_tiles * (p.L + 1) * nch;  // chunks of activations
             long long nu = 0, nv = 0, nh = 0;
@@ -255,60 +261,65 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                 // The epilogue threads wait for one barrier per chunk (a look at an mbarrier costs them a few hundred
                 // cycles): the bytes of the old values are counted on the chunk's own barrier (slot n & 1 = buffer n & 1).
                 // pass >= 1 reads what this CTA stored one pass (nch chunks) earlier
-                if (nh < total_h && (hq < 1 || *stored + unsigned(nch) > unsigned(nh)) &&
-                    mbar_test(smem_u32(&bars->l_free[hp.st]), hp.ph ^ 1u)) {
-                    if (hq >= 1) asm volatile("fence.proxy.async.global;" ::: "memory");
-                    const uint32_t bar = smem_u32(&bars->dh_full[hp.st]);
-                    const uint32_t dst = lbuf_s + hp.st * kHBytesP;
-                    const CUtensorMap* src = hq >= 1 ? &tmY : &tmX;
-                    const int m0 = (cl + ht * ncl) * 2 * kRowsP + hf * kRowsP;
-                    DLP_T(0, hq, hc, 0);
-                    mbar_arrive_expect_tx(bar, kHBytesP);
-                    if (hints) {
-                        const uint64_t pol = hq >= 1 ? pol_h : pol_w;      // x is read once
-                        tma_load_2d_hint(dst, src, col0 + hc * kCWP, m0, bar, pol);
-                        tma_load_2d_hint(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar, pol);
-                    } else {
-                        tma_load_2d(dst, src, col0 + hc * kCWP, m0, bar);
-                        tma_load_2d(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar);
+                if (free_stage(nh < total_h && (hq < 1 || *stored + unsigned(nch) > unsigned(nh)), &bars->l_free[hp.st], hp.ph ^ 1u)) {
+                    if (elect_one()) {
+                        if (hq >= 1) asm volatile("fence.proxy.async.global;" ::: "memory");
+                        const uint32_t bar = smem_u32(&bars->dh_full[hp.st]);
+                        const uint32_t dst = lbuf_s + hp.st * kHBytesP;
+                        const CUtensorMap* src = hq >= 1 ? &tmY : &tmX;
+                        const int m0 = (cl + ht * ncl) * 2 * kRowsP + hf * kRowsP;
+                        DLP_T(0, hq, hc, 0);
+                        mbar_arrive_expect_tx(bar, kHBytesP);
+                        if (hints) {
+                            const uint64_t pol = hq >= 1 ? pol_h : pol_w;      // x is read once
+                            tma_load_2d_hint(dst, src, col0 + hc * kCWP, m0, bar, pol);
+                            tma_load_2d_hint(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar, pol);
+                        } else {
+                            tma_load_2d(dst, src, col0 + hc * kCWP, m0, bar);
+                            tma_load_2d(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar);
+                        }
                     }
-                    hph[hp.st] = int(hp.ph);
+                    __syncwarp();
                     hp.step(kNLP);
                     ++nh;
                     if (++hc == nch) { hc = 0; if (++hq == p.L) { hq = -1; ++ht; } }
                     did = true;
                 }
-                if (nu < total_w && mbar_test(smem_u32(&bars->u_empty[up.st]), up.ph ^ 1u)) {
-                    const uint32_t dst = ubuf_s + up.st * C::U_BYTES;
-                    DLP_T(1, uq, uc, 0);
-                    if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->u_full[up.st]), 2 * C::U_BYTES);
+                if (free_stage(nu < total_w, &bars->u_empty[up.st], up.ph ^ 1u)) {
+                    if (elect_one()) {
+                        const uint32_t dst = ubuf_s + up.st * C::U_BYTES;
+                        DLP_T(1, uq, uc, 0);
+                        if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->u_full[up.st]), 2 * C::U_BYTES);
 #pragma unroll
-                    for (int t = 0; t < C::UT; ++t)
-                        if (hints)
-                            tma_load_2d_pair_hint(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
-                                                  ufull_lead + 8u * up.st, pol_w);
-                        else
-                            tma_load_2d_pair(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
-                                             ufull_lead + 8u * up.st);
-                    uph[up.st] = int(up.ph);
+                        for (int t = 0; t < C::UT; ++t)
+                            if (hints)
+                                tma_load_2d_pair_hint(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
+                                                      ufull_lead + 8u * up.st, pol_w);
+                            else
+                                tma_load_2d_pair(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
+                                                 ufull_lead + 8u * up.st);
+                    }
+                    __syncwarp();
                     up.step(NU);
                     ++nu;
                     if (++uc == nch) { uc = 0; if (++uq == p.L) uq = 0; }
                     did = true;
                 }
-                if (nv < total_w && mbar_test(smem_u32(&bars->v_empty[vp.st]), vp.ph ^ 1u)) {
-                    const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
-                    DLP_T(2, vq - 1, vc, 0);
-                    if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->v_full[vp.st]), 2 * C::V_BYTES);
+                if (free_stage(nv < total_w, &bars->v_empty[vp.st], vp.ph ^ 1u)) {
+                    if (elect_one()) {
+                        const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
+                        DLP_T(2, vq - 1, vc, 0);
+                        if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->v_full[vp.st]), 2 * C::V_BYTES);
 #pragma unroll
-                    for (int t = 0; t < 2; ++t)
-                        if (hints)
-                            tma_load_2d_pair_hint(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
-                                                  vfull_lead + 8u * vp.st, pol_w);
-                        else
-                            tma_load_2d_pair(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
-                                             vfull_lead + 8u * vp.st);
-                    vph[vp.st] = int(vp.ph);
+                        for (int t = 0; t < 2; ++t)
+                            if (hints)
+                                tma_load_2d_pair_hint(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
+                                                      vfull_lead + 8u * vp.st, pol_w);
+                            else
+                                tma_load_2d_pair(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
+                                                 vfull_lead + 8u * vp.st);
+                    }
+                    __syncwarp();
                     vp.step(NV);
                     ++nv;
                     if (++vc == nch) { vc = 0; if (++vq == p.L) vq = 0; }
@@ -316,7 +327,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                 }
                 if (did) {
                     idle = 0;
-                } else if (++idle > p.spin_limit || ((idle & 63u) == 63u && *abort_flag)) {
+                } else if (++idle, __any_sync(0xffffffffu, idle > p.spin_limit || ((idle & 63u) == 63u && *abort_flag))) {
                     err = DLRB200_ERR_TIMEOUT_COPY;
                     err_layer = uq;
                 }
@@ -324,20 +335,20 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
             if (err || *abort_flag) {
                 // copies requested before giving up still land in shared memory: wait for them (the weight copies of
                 // both CTAs are counted in the leader, which the second CTA outlasts through the cluster barrier)
-                for (int i = 0; i < kNLP; ++i)
-                    if (hph[i] >= 0) mbar_wait(smem_u32(&bars->dh_full[i]), uint32_t(hph[i]), kDrainPolls);
+                for (long long m = nh - 1; m >= 0 && m >= nh - kNLP; --m)
+                    mbar_wait(smem_u32(&bars->dh_full[m % kNLP]), uint32_t(m / kNLP) & 1u, kDrainPolls);
                 if (hf == 0) {
-                    for (int i = 0; i < int(NU); ++i)
-                        if (uph[i] >= 0) mbar_wait_cluster(smem_u32(&bars->u_full[i]), uint32_t(uph[i]), kDrainPolls);
-                    for (int i = 0; i < int(NV); ++i)
-                        if (vph[i] >= 0) mbar_wait_cluster(smem_u32(&bars->v_full[i]), uint32_t(vph[i]), kDrainPolls);
+                    for (long long m = nu - 1; m >= 0 && m >= nu - int(NU); --m)
+                        mbar_wait_cluster(smem_u32(&bars->u_full[m % NU]), uint32_t(m / NU) & 1u, kDrainPolls);
+                    for (long long m = nv - 1; m >= 0 && m >= nv - int(NV); --m)
+                        mbar_wait_cluster(smem_u32(&bars->v_full[m % NV]), uint32_t(m / NV) & 1u, kDrainPolls);
                 }
             }
         }
     } else if (warp == 1) {
         // =============================== U-MMA warp (leader) =======================
         // buffer = s(q)[256 x R] * U'[q][chunk rows, :]^T, A from tensor memory of both CTAs
-        if (hf == 0 && elect_one()) {
+        if (hf == 0) {
             constexpr uint32_t idesc_u = umma_idesc_bf16(256, kCWP);
             RingPos up;
             uint32_t n = 0;
@@ -347,46 +358,51 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                 // chunk's barrier gets its commit (which arrives at once) when the buffer is free
                 for (int c = 0; c < nch && !err; ++c, ++n) {
                     const uint32_t b = n & 1u;
-                    if (!w.cta(smem_u32(&bars->a_free[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
-                    umma_commit2_mask(smem_u32(&bars->dh_full[b]), pair_mask);
+                    if (!wait_cta(smem_u32(&bars->a_free[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (elect_one()) umma_commit2_mask(smem_u32(&bars->dh_full[b]), pair_mask);
+                    __syncwarp();
                 }
                 for (int q = 0; q < p.L && !err; ++q) {
                     err_layer = q;
                     DLP_T(3, q, 0, 7);
-                    if (!w.cluster(smem_u32(&bars->s_ready), c_s & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cluster(smem_u32(&bars->s_ready), c_s & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     DLP_T(3, q, 0, 0);
                     ++c_s;
                     tc_fence_after();
                     for (int c = 0; c < nch; ++c, ++n) {
                         const uint32_t b = n & 1u;
                         // the weights land early: wait for them first, off the critical path
-                        if (!w.cluster(smem_u32(&bars->u_full[up.st]), up.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                        if (!wait_cluster(smem_u32(&bars->u_full[up.st]), up.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                         DLP_T(3, q, c, 1);
                         const uint32_t acc = tmem_base + kBufCol + b * 128u;
                         // the buffer is free once the V contraction of the chunk two before has read it
-                        if (!w.cta(smem_u32(&bars->a_free[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (!wait_cta(smem_u32(&bars->a_free[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         DLP_T(3, q, c, 2);
                         tc_fence_after();
                         const uint32_t ub = ubuf_s + up.st * C::U_BYTES;
+                        if (elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < R / 16; ++k) {
-                            const uint64_t bdesc = umma_desc(ub + uint32_t(k / 4) * C::U_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
-                            umma_ts2(acc, tmem_base + kSCol + uint32_t(8 * k), bdesc, idesc_u, k ? 1u : 0u);
+                            for (int k = 0; k < R / 16; ++k) {
+                                const uint64_t bdesc = umma_desc(ub + uint32_t(k / 4) * C::U_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
+                                umma_ts2(acc, tmem_base + kSCol + uint32_t(8 * k), bdesc, idesc_u, k ? 1u : 0u);
+                            }
+                            umma_commit2_mask(smem_u32(&bars->u_empty[up.st]), pair_mask);
+                            umma_commit2_mask(smem_u32(&bars->dh_full[b]), pair_mask);
                         }
-                        umma_commit2_mask(smem_u32(&bars->u_empty[up.st]), pair_mask);
+                        __syncwarp();
                         up.step(NU);
-                        umma_commit2_mask(smem_u32(&bars->dh_full[b]), pair_mask);
                         DLP_T(3, q, c, 3);
                     }
                 }
             }
-            umma_commit2(smem_u32(&bars->drain[0]));
+            if (elect_one()) umma_commit2(smem_u32(&bars->drain[0]));
+            __syncwarp();
             mbar_wait(smem_u32(&bars->drain[0]), 0, kDrainPolls);
         }
     } else if (warp == 2) {
         // =============================== V-MMA warp (leader) =======================
         // z(q+1)[256 x R] += h_new[chunk][256 x 128] * V'[q+1][:, chunk]^T, A = the updated chunk in tensor memory
-        if (hf == 0 && elect_one()) {
+        if (hf == 0) {
             constexpr uint32_t idesc_v = umma_idesc_bf16(256, R);
             RingPos vp;
             uint32_t n = 0;
@@ -397,31 +413,37 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     for (int c = 0; c < nch; ++c, ++n) {
                         const uint32_t b = n & 1u;
                         // the weights land early: wait for them first, off the critical path
-                        if (feeds && !w.cluster(smem_u32(&bars->v_full[vp.st]), vp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                        if (feeds && !wait_cluster(smem_u32(&bars->v_full[vp.st]), vp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                         DLP_T(4, q, c, 1);
-                        if (!w.cluster(smem_u32(&bars->a_ready[b]), (n >> 1) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (!wait_cluster(smem_u32(&bars->a_ready[b]), (n >> 1) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         DLP_T(4, q, c, 2);
                         tc_fence_after();
                         if (feeds) {
                             const uint32_t a0 = tmem_base + kBufCol + b * 128u;
                             const uint32_t vb = vbuf_s + vp.st * C::V_BYTES;
+                            if (elect_one()) {
 #pragma unroll
-                            for (int k = 0; k < kCWP / 16; ++k) {
-                                const uint64_t bdesc = umma_desc(vb + uint32_t(k / 4) * C::V_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
-                                umma_ts2(tmem_base + kZCol, a0 + uint32_t(32 * (k / 2) + 8 * (k % 2)), bdesc, idesc_v, (c | k) ? 1u : 0u);
+                                for (int k = 0; k < kCWP / 16; ++k) {
+                                    const uint64_t bdesc = umma_desc(vb + uint32_t(k / 4) * C::V_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
+                                    umma_ts2(tmem_base + kZCol, a0 + uint32_t(32 * (k / 2) + 8 * (k % 2)), bdesc, idesc_v, (c | k) ? 1u : 0u);
+                                }
+                                umma_commit2_mask(smem_u32(&bars->v_empty[vp.st]), pair_mask);
+                                umma_commit2_mask(smem_u32(&bars->a_free[b]), pair_mask);       // the chunk has been read
                             }
-                            umma_commit2_mask(smem_u32(&bars->v_empty[vp.st]), pair_mask);
                             vp.step(NV);
+                        } else if (elect_one()) {
+                            umma_commit2_mask(smem_u32(&bars->a_free[b]), pair_mask);   // last layer: nothing reads it, arrives at once
                         }
-                        // the chunk has been read (last layer: nothing reads it, the commit arrives at once)
-                        umma_commit2_mask(smem_u32(&bars->a_free[b]), pair_mask);
+                        __syncwarp();
                         DLP_T(4, q, c, 3);
                     }
                     if (err) break;
-                    if (feeds) umma_commit2_mask(smem_u32(&bars->z_full), pair_mask);
+                    if (feeds && elect_one()) umma_commit2_mask(smem_u32(&bars->z_full), pair_mask);
+                    __syncwarp();
                 }
             }
-            umma_commit2(smem_u32(&bars->drain[1]));
+            if (elect_one()) umma_commit2(smem_u32(&bars->drain[1]));
+            __syncwarp();
             mbar_wait(smem_u32(&bars->drain[1]), 0, kDrainPolls);
         }
     } else if (warp == 3) {
@@ -429,14 +451,17 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         // new chunk -> output buffer.  A slot is released when the copy has read it; the chunk counts as
         // stored (readable by the next pass) once its bulk group is complete, which is checked two chunks late
         // so that this warp never waits for a write in flight.
-        if (lane == 0) {
+        {
             RingPos sp;
             const uint64_t pol_h = l2_policy_evict_last(), pol_out = l2_policy_evict_first();
             const bool hints = !(PROF && (p.exp & 32));
             unsigned int n = 0;              // chunks seen (all tiles, all passes): the producer counts the same way
             // the store slots of the first two chunks are free from the start
-            mbar_arrive(smem_u32(&bars->dh_full[0]));
-            mbar_arrive(smem_u32(&bars->dh_full[1]));
+            if (lane == 0) {
+                mbar_arrive(smem_u32(&bars->dh_full[0]));
+                mbar_arrive(smem_u32(&bars->dh_full[1]));
+            }
+            __syncwarp();
             for (int t = 0; t < my_tiles && !err; ++t) {
                 const int m0 = (cl + t * ncl) * 2 * kRowsP + hf * kRowsP;
                 // (the pass over x stores nothing but walks the slots like the others: chunk n uses slot n & 1, as it
@@ -444,31 +469,34 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                 for (int q = -1; q < p.L && !err; ++q) {
                     err_layer = q;
                     for (int c = 0; c < nch; ++c, ++n) {
-                        if (!w.cta(smem_u32(&bars->s_written[sp.st]), sp.ph)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
-                        DLP_T(5, q, c, 0);
-                        if (q >= 0 && m0 < p.M && !(PROF && (p.exp & 8))) {   // a CTA whose rows lie wholly past the batch stores nothing
-                            const uint32_t src = sbuf_s + sp.st * kHBytesP;
-                            if (hints) {       // the last layer's output is not read again here: first to leave L2
-                                const uint64_t pol = q + 1 < p.L ? pol_h : pol_out;
-                                tma_store_2d_hint(&tmY, col0 + c * kCWP, m0, src, pol);
-                                tma_store_2d_hint(&tmY, col0 + c * kCWP + 64, m0, src + 16384, pol);
-                            } else {
-                                tma_store_2d(&tmY, col0 + c * kCWP, m0, src);
-                                tma_store_2d(&tmY, col0 + c * kCWP + 64, m0, src + 16384);
+                        if (!wait_cta(smem_u32(&bars->s_written[sp.st]), sp.ph)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (lane == 0) {           // (bulk groups belong to a thread)
+                            DLP_T(5, q, c, 0);
+                            if (q >= 0 && m0 < p.M && !(PROF && (p.exp & 8))) {   // a CTA whose rows lie wholly past the batch stores nothing
+                                const uint32_t src = sbuf_s + sp.st * kHBytesP;
+                                if (hints) {       // the last layer's output is not read again here: first to leave L2
+                                    const uint64_t pol = q + 1 < p.L ? pol_h : pol_out;
+                                    tma_store_2d_hint(&tmY, col0 + c * kCWP, m0, src, pol);
+                                    tma_store_2d_hint(&tmY, col0 + c * kCWP + 64, m0, src + 16384, pol);
+                                } else {
+                                    tma_store_2d(&tmY, col0 + c * kCWP, m0, src);
+                                    tma_store_2d(&tmY, col0 + c * kCWP + 64, m0, src + 16384);
+                                }
                             }
+                            bulk_commit_group();
+                            bulk_wait_group_read<0>();
+                            DLP_T(5, q, c, 1);
+                            // the slot is free for the chunk after next: one of the three arrivals its barrier waits for
+                            mbar_arrive(smem_u32(&bars->dh_full[sp.st]));
+                            bulk_wait_group<2>();            // every group but the last two is complete
+                            if (n + 1u > *stored + 2u) *stored = n + 1u - 2u;
                         }
-                        bulk_commit_group();
-                        bulk_wait_group_read<0>();
-                        DLP_T(5, q, c, 1);
-                        // the slot is free for the chunk after next: one of the three arrivals its barrier waits for
-                        mbar_arrive(smem_u32(&bars->dh_full[sp.st]));
+                        __syncwarp();
                         sp.step(kNSP);
-                        bulk_wait_group<2>();            // every group but the last two is complete
-                        if (n + 1u > *stored + 2u) *stored = n + 1u - 2u;
                     }
                 }
             }
-            bulk_wait_group<0>();
+            if (lane == 0) bulk_wait_group<0>();
         }
     } else if (warp >= 4) {
         // =============================== epilogue warps =============================
@@ -509,7 +537,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     DLP_TE(q, c, 0);
                     // ---- the one wait of a chunk: dh is in the buffer (in the pass over x: the buffer is free), the old
                     // values of the chunk have landed in their slot and the store slot is free
-                    if (!w.cta(smem_u32(&bars->dh_full[b]), (n >> 1) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cta(smem_u32(&bars->dh_full[b]), (n >> 1) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     tc_fence_after();
                     DLP_TE(q, c, 1);
                     uint32_t cur[16];
@@ -587,7 +615,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     float ssq = ssq0 + ssq1;
                     ssq0 = ssq1 = 0.f;
                     DLP_TE(q, 24, 0);
-                    if (!w.cluster(smem_u32(&bars->z_full), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cluster(smem_u32(&bars->z_full), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     DLP_TE(q, 24, 1);
                     tc_fence_after();
                     uint32_t zv[NZ];
@@ -602,13 +630,13 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                         const uint32_t partner = crank ^ (2u << step);
                         if (step == 0) {
                             // the first partner acknowledged the last message of the layer before
-                            if (c_z > 0 && !w.cluster(smem_u32(&bars->xack_bar[0]), (c_z - 1u) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                            if (c_z > 0 && !wait_cluster(smem_u32(&bars->xack_bar[0]), (c_z - 1u) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         } else {
                             // this CTA has read the message of the step before: the partner of this step may send; and
                             // that partner must have read its own
                             __syncwarp();
                             if (lane == 0) mbar_arrive_remote_light(mapa(smem_u32(&bars->xack_bar[step]), partner));
-                            if (!w.cluster(smem_u32(&bars->xack_bar[step]), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                            if (!wait_cluster(smem_u32(&bars->xack_bar[step]), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         }
                         const uint32_t p_recv = mapa(smem_u32(recv), partner);
                         const uint32_t p_recv_q = mapa(smem_u32(recv_q), partner);
@@ -628,7 +656,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                         }
                         st_async_b32(p_recv_q + uint32_t(et * 4), __float_as_uint(ssq), p_xchg);
                         DLP_TE(q, 24, 2);
-                        if (!w.cluster(smem_u32(&bars->xchg_bar[step]), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (!wait_cluster(smem_u32(&bars->xchg_bar[step]), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         DLP_TE(q, 24, 3);
                         ssq += recv_q[et];
 #pragma unroll
@@ -645,7 +673,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     ssqx[cq * kRowsP + er] = ssq;              // index et: the word this thread's received partial came in
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bars->ssq_bar));
-                    if (!w.cta(smem_u32(&bars->ssq_bar), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cta(smem_u32(&bars->ssq_bar), c_z & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     // the four quarters in a fixed order: every thread of a row gets the same total
                     const float tot = (ssqx[er] + ssqx[kRowsP + er]) + (ssqx[2 * kRowsP + er] + ssqx[3 * kRowsP + er]);
                     const float rstd = rsqrtf(tot * p.inv_d + p.eps);
@@ -703,7 +731,7 @@ PairShape pick_shape(int num_tiles, int d, int r, const int (&max_clusters)[3], 
     int forced = 0;
     if (const char* e = getenv("DLRB200_PAIR_SPLIT")) forced = atoi(e);
     const int nch = d / kCWP;
-    const double t_chunk = r == 128 ? 1.09 : 0.80;
+    const double t_chunk = r == 128 ? 0.98 : 0.85;
     const size_t tile_bytes = size_t(2 * kRowsP) * d * 2;
     int fit = int(double(l2_bytes) * 0.62 / double(tile_bytes));      // tiles whose rows stay in L2 beside the weight stream
     if (fit < 1) fit = 1;
@@ -715,7 +743,7 @@ PairShape pick_shape(int num_tiles, int d, int r, const int (&max_clusters)[3], 
         int clusters = max_clusters[i] < fit ? max_clusters[i] : fit;
         if (clusters > num_tiles) clusters = num_tiles;
         const int rounds = (num_tiles + clusters - 1) / clusters;
-        const double pause = (r == 128 ? 3.4 : 2.0) + (pp == 4 ? 2.8 : (pp == 2 ? 1.0 : 0.0));
+        const double pause = (r == 128 ? 3.6 : 1.8) + (pp == 4 ? (r == 128 ? 1.4 : 1.9) : (pp == 2 ? 1.0 : 0.0));
         const double t = rounds * ((nch / pp) * t_chunk + pause);
         if (t < best_t) { best_t = t; best = PairShape{pp, clusters}; }
     }
