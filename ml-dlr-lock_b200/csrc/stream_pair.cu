@@ -23,9 +23,9 @@
 // each SM's port halve; nothing is multicast, each CTA loads its own half with
 // a plain TMA load whose bytes are counted on the leader's barrier.
 //
-// Roles per CTA (640 threads): TMA producer, U-MMA issuer and V-MMA issuer
-// (these two work in the leader, the even-ranked CTA of the pair, only), store
-// warp (owns tensor memory), 16 epilogue warps.  The epilogue warps of the
+// Roles per CTA (704 threads): three TMA producers (activations, U', V'), U-MMA
+// issuer and V-MMA issuer (these two work in the leader, the even-ranked CTA of
+// the pair, only), store warp (owns tensor memory), 16 epilogue warps.  The epilogue warps of the
 // second CTA signal the leader's barriers with remote arrives; the leader's
 // tcgen05.commit signals the barriers of both CTAs.
 //
@@ -41,6 +41,8 @@
 // Every role waits as a whole warp and elects a lane for what one thread does (a
 // look at a barrier by one lane of a split warp costs about 250 cycles): d = 4096,
 // 8192 rows, back to back: 3.27 ms with one thread per role, 2.97 ms so.
+// Each of the three copy streams has a warp: one warp for all took about 1600 cycles
+// for the six requests of a chunk and was the slowest role (3.06 ms then, 2.83 ms so).
 //
 // All waits are bounded; a wait that gives up raises an abort flag, records a
 // status word and every role drains and leaves.
@@ -60,7 +62,9 @@ constexpr int kRowsP = 128;              // rows per CTA (a pair: 256)
 constexpr int kCWP = 128;                // columns per chunk
 constexpr int kEpiWarpsP = 16;           // four threads per row: each owns 32 of a chunk's 128 columns
 constexpr int kEpiThreadsP = kEpiWarpsP * 32;
-constexpr int kThreadsP = 128 + kEpiThreadsP;   // 20 warps: producer, U-MMA, V-MMA, store (owns tensor memory), 16 epilogue
+constexpr int kWarpU = 4 + kEpiWarpsP, kWarpV = kWarpU + 1;   // weight producers
+// 22 warps: producer of activations, U-MMA, V-MMA, store (owns tensor memory), 16 epilogue, producers of U' and V'
+constexpr int kThreadsP = 128 + kEpiThreadsP + 64;
 constexpr int kMaxWP = 4;                // most stages of a weight ring
 constexpr int kNLP = 2;                  // slots the old values of a chunk are loaded into
 constexpr int kNSP = 2;                  // slots the new values are written to and stored from
@@ -238,112 +242,132 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     // A pass q = -1 .. L-1 walks the nch chunks once.  Pass q >= 0 applies the update of layer q; pass q < L-1
     // feeds the V contraction of layer q+1.  Chunk number n (all tiles, all passes) uses buffer n & 1.
     if (warp == 0) {
-        // =============================== TMA producer ===============================
-        // (the whole warp looks at the barriers, one lane issues: see mbar_wait_warp)
+        // =============================== TMA producer: activations ==================
         {
-            RingPos up, vp, hp;
-            auto free_stage = [&](bool want, uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, want && mbar_test(smem_u32(bar), parity)) != 0; };
-            const long long total_w = (long long)my_tiles * p.L * nch;        // stages of each weight stream
+            RingPos hp;
             const long long total_h = (long long)my_tiles * (p.L + 1) * nch;  // chunks of activations
-            long long nu = 0, nv = 0, nh = 0;
-            int uq = 0, uc = 0, vq = 0, vc = 0;
+            long long nh = 0;
             int ht = 0, hq = -1, hc = 0;
-            uint32_t idle = 0;
-            // the weight stages of both CTAs are counted on the leader's barriers
-            const uint32_t ufull_lead = mapa(smem_u32(&bars->u_full[0]), lead);
-            const uint32_t vfull_lead = mapa(smem_u32(&bars->v_full[0]), lead);
             // the weights pass through L2 once per cluster and layer, the activations come back every layer: tell
             // L2 which to keep (without the hints over half of every layer's output is written back to DRAM)
             const uint64_t pol_w = l2_policy_evict_first(), pol_h = l2_policy_evict_last();
             const bool hints = !(PROF && (p.exp & 32));
-            while ((nu < total_w || nv < total_w || nh < total_h) && !err) {
-                bool did = false;
+            while (nh < total_h && !err) {
+                err_layer = hq < 0 ? 0 : hq;
                 // The epilogue threads wait for one barrier per chunk (a look at an mbarrier costs them a few hundred
                 // cycles): the bytes of the old values are counted on the chunk's own barrier (slot n & 1 = buffer n & 1).
                 // pass >= 1 reads what this CTA stored one pass (nch chunks) earlier
-                if (free_stage(nh < total_h && (hq < 1 || *stored + unsigned(nch) > unsigned(nh)), &bars->l_free[hp.st], hp.ph ^ 1u)) {
-                    if (elect_one()) {
-                        if (hq >= 1) asm volatile("fence.proxy.async.global;" ::: "memory");
-                        const uint32_t bar = smem_u32(&bars->dh_full[hp.st]);
-                        const uint32_t dst = lbuf_s + hp.st * kHBytesP;
-                        const CUtensorMap* src = hq >= 1 ? &tmY : &tmX;
-                        const int m0 = (cl + ht * ncl) * 2 * kRowsP + hf * kRowsP;
-                        DLP_T(0, hq, hc, 0);
-                        mbar_arrive_expect_tx(bar, kHBytesP);
-                        if (hints) {
-                            const uint64_t pol = hq >= 1 ? pol_h : pol_w;      // x is read once
-                            tma_load_2d_hint(dst, src, col0 + hc * kCWP, m0, bar, pol);
-                            tma_load_2d_hint(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar, pol);
-                        } else {
-                            tma_load_2d(dst, src, col0 + hc * kCWP, m0, bar);
-                            tma_load_2d(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar);
-                        }
+                if (hq >= 1) {
+                    uint32_t idle = 0;
+                    while (!__all_sync(0xffffffffu, *stored + unsigned(nch) > unsigned(nh))) {
+                        ++idle;
+                        if (__any_sync(0xffffffffu, idle > p.spin_limit || ((idle & 63u) == 63u && *abort_flag))) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                     }
-                    __syncwarp();
-                    hp.step(kNLP);
-                    ++nh;
-                    if (++hc == nch) { hc = 0; if (++hq == p.L) { hq = -1; ++ht; } }
-                    did = true;
+                    if (err) break;
                 }
-                if (free_stage(nu < total_w, &bars->u_empty[up.st], up.ph ^ 1u)) {
-                    if (elect_one()) {
-                        const uint32_t dst = ubuf_s + up.st * C::U_BYTES;
-                        DLP_T(1, uq, uc, 0);
-                        if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->u_full[up.st]), 2 * C::U_BYTES);
-#pragma unroll
-                        for (int t = 0; t < C::UT; ++t)
-                            if (hints)
-                                tma_load_2d_pair_hint(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
-                                                      ufull_lead + 8u * up.st, pol_w);
-                            else
-                                tma_load_2d_pair(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
-                                                 ufull_lead + 8u * up.st);
+                if (!wait_cta(smem_u32(&bars->l_free[hp.st]), hp.ph ^ 1u)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                if (elect_one()) {
+                    if (hq >= 1) asm volatile("fence.proxy.async.global;" ::: "memory");
+                    const uint32_t bar = smem_u32(&bars->dh_full[hp.st]);
+                    const uint32_t dst = lbuf_s + hp.st * kHBytesP;
+                    const CUtensorMap* src = hq >= 1 ? &tmY : &tmX;
+                    const int m0 = (cl + ht * ncl) * 2 * kRowsP + hf * kRowsP;
+                    DLP_T(0, hq, hc, 0);
+                    mbar_arrive_expect_tx(bar, kHBytesP);
+                    if (hints) {
+                        const uint64_t pol = hq >= 1 ? pol_h : pol_w;      // x is read once
+                        tma_load_2d_hint(dst, src, col0 + hc * kCWP, m0, bar, pol);
+                        tma_load_2d_hint(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar, pol);
+                    } else {
+                        tma_load_2d(dst, src, col0 + hc * kCWP, m0, bar);
+                        tma_load_2d(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar);
                     }
-                    __syncwarp();
-                    up.step(NU);
-                    ++nu;
-                    if (++uc == nch) { uc = 0; if (++uq == p.L) uq = 0; }
-                    did = true;
                 }
-                if (free_stage(nv < total_w, &bars->v_empty[vp.st], vp.ph ^ 1u)) {
-                    if (elect_one()) {
-                        const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
-                        DLP_T(2, vq - 1, vc, 0);
-                        if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->v_full[vp.st]), 2 * C::V_BYTES);
-#pragma unroll
-                        for (int t = 0; t < 2; ++t)
-                            if (hints)
-                                tma_load_2d_pair_hint(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
-                                                      vfull_lead + 8u * vp.st, pol_w);
-                            else
-                                tma_load_2d_pair(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
-                                                 vfull_lead + 8u * vp.st);
-                    }
-                    __syncwarp();
-                    vp.step(NV);
-                    ++nv;
-                    if (++vc == nch) { vc = 0; if (++vq == p.L) vq = 0; }
-                    did = true;
-                }
-                if (did) {
-                    idle = 0;
-                } else if (++idle, __any_sync(0xffffffffu, idle > p.spin_limit || ((idle & 63u) == 63u && *abort_flag))) {
-                    err = DLRB200_ERR_TIMEOUT_COPY;
-                    err_layer = uq;
-                }
+                __syncwarp();
+                hp.step(kNLP);
+                ++nh;
+                if (++hc == nch) { hc = 0; if (++hq == p.L) { hq = -1; ++ht; } }
             }
-            if (err || *abort_flag) {
-                // copies requested before giving up still land in shared memory: wait for them (the weight copies of
-                // both CTAs are counted in the leader, which the second CTA outlasts through the cluster barrier)
+            // copies requested before giving up still land in shared memory: wait for them
+            if (err || *abort_flag)
                 for (long long m = nh - 1; m >= 0 && m >= nh - kNLP; --m)
                     mbar_wait(smem_u32(&bars->dh_full[m % kNLP]), uint32_t(m / kNLP) & 1u, kDrainPolls);
-                if (hf == 0) {
-                    for (long long m = nu - 1; m >= 0 && m >= nu - int(NU); --m)
-                        mbar_wait_cluster(smem_u32(&bars->u_full[m % NU]), uint32_t(m / NU) & 1u, kDrainPolls);
-                    for (long long m = nv - 1; m >= 0 && m >= nv - int(NV); --m)
-                        mbar_wait_cluster(smem_u32(&bars->v_full[m % NV]), uint32_t(m / NV) & 1u, kDrainPolls);
+        }
+    } else if (warp == kWarpU) {
+        // =============================== TMA producer: U' ==========================
+        {
+            RingPos up;
+            const long long total_w = (long long)my_tiles * p.L * nch;
+            long long nu = 0;
+            int uq = 0, uc = 0;
+            // the weight stages of both CTAs are counted on the leader's barriers
+            const uint32_t ufull_lead = mapa(smem_u32(&bars->u_full[0]), lead);
+            const uint64_t pol_w = l2_policy_evict_first();
+            const bool hints = !(PROF && (p.exp & 32));
+            while (nu < total_w && !err) {
+                err_layer = uq;
+                if (!wait_cta(smem_u32(&bars->u_empty[up.st]), up.ph ^ 1u)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                if (elect_one()) {
+                    const uint32_t dst = ubuf_s + up.st * C::U_BYTES;
+                    DLP_T(1, uq, uc, 0);
+                    if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->u_full[up.st]), 2 * C::U_BYTES);
+#pragma unroll
+                    for (int t = 0; t < C::UT; ++t)
+                        if (hints)
+                            tma_load_2d_pair_hint(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
+                                                  ufull_lead + 8u * up.st, pol_w);
+                        else
+                            tma_load_2d_pair(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
+                                             ufull_lead + 8u * up.st);
                 }
+                __syncwarp();
+                up.step(NU);
+                ++nu;
+                if (++uc == nch) { uc = 0; if (++uq == p.L) uq = 0; }
             }
+            // (the weight copies of both CTAs are counted in the leader, which the second CTA outlasts through the cluster
+            // barrier)
+            if ((err || *abort_flag) && hf == 0)
+                for (long long m = nu - 1; m >= 0 && m >= nu - int(NU); --m)
+                    mbar_wait_cluster(smem_u32(&bars->u_full[m % NU]), uint32_t(m / NU) & 1u, kDrainPolls);
+        }
+    } else if (warp == kWarpV) {
+        // =============================== TMA producer: V' ==========================
+        {
+            RingPos vp;
+            const long long total_w = (long long)my_tiles * p.L * nch;
+            long long nv = 0;
+            int vq = 0, vc = 0;
+            // the weight stages of both CTAs are counted on the leader's barriers
+            const uint32_t vfull_lead = mapa(smem_u32(&bars->v_full[0]), lead);
+            const uint64_t pol_w = l2_policy_evict_first();
+            const bool hints = !(PROF && (p.exp & 32));
+            while (nv < total_w && !err) {
+                err_layer = vq;
+                if (!wait_cta(smem_u32(&bars->v_empty[vp.st]), vp.ph ^ 1u)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
+                if (elect_one()) {
+                    const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
+                    DLP_T(2, vq - 1, vc, 0);
+                    if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->v_full[vp.st]), 2 * C::V_BYTES);
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+                        if (hints)
+                            tma_load_2d_pair_hint(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
+                                                  vfull_lead + 8u * vp.st, pol_w);
+                        else
+                            tma_load_2d_pair(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
+                                             vfull_lead + 8u * vp.st);
+                }
+                __syncwarp();
+                vp.step(NV);
+                ++nv;
+                if (++vc == nch) { vc = 0; if (++vq == p.L) vq = 0; }
+            }
+            // (the weight copies of both CTAs are counted in the leader, which the second CTA outlasts through the cluster
+            // barrier)
+            if ((err || *abort_flag) && hf == 0)
+                for (long long m = nv - 1; m >= 0 && m >= nv - int(NV); --m)
+                    mbar_wait_cluster(smem_u32(&bars->v_full[m % NV]), uint32_t(m / NV) & 1u, kDrainPolls);
         }
     } else if (warp == 1) {
         // =============================== U-MMA warp (leader) =======================
