@@ -5,7 +5,7 @@
 //
 // Same data flow as the one-CTA streamed kernel (stream.cu): rows are
 // independent (dlr_lock/model.py:96-100 acts on each token alone), the
-// activations stream chunk by chunk (128 columns) through a staging slot in
+// activations stream chunk by chunk (64 columns) through a staging slot in
 // shared memory and through tensor memory, in place in the output buffer, and
 // the two contractions of neighbouring layers run interleaved,
 //     dh        = s(l) * U'[l][chunk]^T          (U-MMA)
@@ -59,34 +59,36 @@ namespace dlr {
 namespace {
 
 constexpr int kRowsP = 128;              // rows per CTA (a pair: 256)
-constexpr int kCWP = 128;                // columns per chunk
-constexpr int kEpiWarpsP = 16;           // four threads per row: each owns 32 of a chunk's 128 columns
+constexpr int kCWP = 64;                 // columns per chunk
+constexpr int kEpiWarpsP = 16;           // two groups of 8: two threads per row, each with 32 of a chunk's 64 columns
+constexpr int kBufs = 4;                 // chunks in flight: dh buffers, load slots and store slots
 constexpr int kEpiThreadsP = kEpiWarpsP * 32;
 constexpr int kWarpU = 4 + kEpiWarpsP, kWarpV = kWarpU + 1;   // weight producers
 // 22 warps: producer of activations, U-MMA, V-MMA, store (owns tensor memory), 16 epilogue, producers of U' and V'
 constexpr int kThreadsP = 128 + kEpiThreadsP + 64;
-constexpr int kMaxWP = 4;                // most stages of a weight ring
-constexpr int kNLP = 2;                  // slots the old values of a chunk are loaded into
-constexpr int kNSP = 2;                  // slots the new values are written to and stored from
-constexpr int kHBytesP = 2 * 16384;      // one chunk: two tiles of 128 rows x 64 columns (128-byte swizzle)
+constexpr int kMaxWP = 8;                // most stages of a weight ring
+constexpr int kStoreLag = 4;             // a chunk counts as stored this many chunks late
+constexpr int kHBytesP = 16384;          // one chunk: a tile of 128 rows x 64 columns (128-byte swizzle)
 
-// Tensor-memory columns (per CTA): z [0, R) | s [128, 128 + R/2) | buffer 0 [256, 384) | buffer 1 [384, 512).
-// A buffer first holds dh of a chunk (fp32, 128 columns); the epilogue thread that has read its 32 columns of
+// Tensor-memory columns (per CTA): z [0, R) | s [128, 128 + R/2) | four buffers of 64 columns [256, 512).
+// A buffer first holds dh of a chunk (fp32, 64 columns); the epilogue thread that has read its 32 columns of
 // dh writes its 32 updated values back as bf16 over the first 16 of them, and the V contraction reads the
 // chunk from there (K step k: columns 32 (k / 2) + 8 (k % 2)).  The chunk therefore needs no buffer of its
-// own, two chunks are in flight, and the epilogue never waits for the V contraction of the chunk before.
+// own, and four chunks are in flight: what bounds a chunk is the chain U contraction, epilogue, V contraction
+// with a signal between each two, of which the tensor core works a third.  Against two chunks of 128 columns in
+// flight (ms): d = 4096, 2048 rows 1.65 / 1.59, 8192 rows 2.83 / 2.79; d = 2048, 2000 rows 0.99 / 0.91; d = 1024,
+// r = 128, 4000 rows 0.81 / 0.72.
 template <int R>
 struct PCfg {
     static constexpr uint32_t Z_COL = 0, S_COL = 128, BUF_COL = 256;
-    // this CTA's half of a chunk's U' rows: 64 rows x R K-columns, in tiles of 64 K-columns
+    // this CTA's half of a chunk's U' rows: 32 rows x R K-columns, in tiles of 64 K-columns
     static constexpr int UT = R / 64;
-    static constexpr int U_TILE_BYTES = 64 * 128;
+    static constexpr int U_TILE_BYTES = (kCWP / 2) * 128;
     static constexpr int U_BYTES = UT * U_TILE_BYTES;
-    // this CTA's half of V'[l]: R/2 rows x the chunk's 128 K-columns, in two tiles of 64 K-columns
-    static constexpr int V_TILE_BYTES = (R / 2) * 128;
-    static constexpr int V_BYTES = 2 * V_TILE_BYTES;
-    static constexpr int NU = R == 128 ? 2 : 4;
-    static constexpr int NV = R == 128 ? 2 : 4;
+    // this CTA's half of V'[l]: R/2 rows x the chunk's 64 K-columns
+    static constexpr int V_BYTES = (R / 2) * 128;
+    static constexpr int NU = R == 128 ? 4 : 8;
+    static constexpr int NV = R == 128 ? 4 : 8;
     // message of one thread to a partner pair: its R/4 columns of z as bf16 (NZW words of 16 bytes) and its
     // partial sum of squares (4 bytes)
     static constexpr int NZ = R / 4;
@@ -94,23 +96,23 @@ struct PCfg {
     static constexpr int RECV_Z_BYTES = NZW * kEpiThreadsP * 16;
     static constexpr int RECV_BYTES = RECV_Z_BYTES + kEpiThreadsP * 4;
     // the partial sums of squares of this CTA are added in place onto the received ones: no array of their own
-    static constexpr int SMEM_BYTES = (kNLP + kNSP) * kHBytesP + NU * U_BYTES + NV * V_BYTES + RECV_BYTES + 512 /*barriers*/;
+    static constexpr int SMEM_BYTES = (kBufs + kBufs) * kHBytesP + NU * U_BYTES + NV * V_BYTES + RECV_BYTES + 512 /*barriers*/;
 };
 
 struct PBars {
     uint64_t u_full[kMaxWP], u_empty[kMaxWP];   // full: in the leader, bytes of both CTAs; empty: commit, both CTAs
     uint64_t v_full[kMaxWP], v_empty[kMaxWP];
-    uint64_t l_free[kNLP];       // the 16 epilogue warps have it in registers
-    uint64_t s_written[kNSP];    // the 16 epilogue warps have written the new chunk
+    uint64_t l_free[kBufs];      // the 8 epilogue warps of the chunk have it in registers
+    uint64_t s_written[kBufs];   // the 8 epilogue warps have written the new chunk
     // The one barrier an epilogue thread waits for per chunk (a look at an mbarrier costs a few hundred cycles even
     // when its phase is complete, and the epilogue is on the loop that bounds the time per chunk).  Chunk n uses
-    // buffer, load slot and store slot n & 1, and barrier [n & 1] collects three arrivals: the commit of the U
+    // buffer, load slot and store slot n % 4, and barrier [n % 4] collects three arrivals: the commit of the U
     // contraction (both CTAs; in the pass over x an empty commit once the buffer is free), the producer's arrival
     // that carries the byte count of the old values, and the store warp's arrival when the bulk store of the chunk
-    // two before has read the store slot.
-    uint64_t dh_full[2];
-    uint64_t a_ready[2];         // leader: the 32 epilogue warps have put the updated chunk (bf16) into the buffer
-    uint64_t a_free[2];          // commit, both CTAs: the V contraction has read the chunk, the buffer is free
+    // four before has read the store slot.
+    uint64_t dh_full[kBufs];
+    uint64_t a_ready[kBufs];     // leader: the 16 epilogue warps of the chunk have put the updated chunk (bf16) into the buffer
+    uint64_t a_free[kBufs];      // commit, both CTAs: the V contraction has read the chunk, the buffer is free
     uint64_t z_full;             // commit, both CTAs
     uint64_t s_ready;            // leader: 32 epilogue warps
     uint64_t xchg_bar[2];        // per exchange step: the partner's message has arrived (bytes)
@@ -126,7 +128,7 @@ static_assert(sizeof(PBars) <= 512, "barrier block");
 
 struct PParams {
     int M, d, L;
-    int nch;                  // chunks per row: d / 128
+    int nch;                  // chunks per row: d / 64
     int pp;                   // pairs per cluster (1, 2 or 4), each with nch / pp of the chunks
     int num_tiles;            // 256-row tiles
     float eps, inv_d;
@@ -157,8 +159,8 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     // the swizzled tiles need a 1024-byte aligned base: asked for here, checked below
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* lbuf = smem;
-    uint8_t* sbuf = lbuf + kNLP * kHBytesP;
-    uint8_t* ubuf = sbuf + kNSP * kHBytesP;
+    uint8_t* sbuf = lbuf + kBufs * kHBytesP;
+    uint8_t* ubuf = sbuf + kBufs * kHBytesP;
     uint8_t* vbuf = ubuf + NU * C::U_BYTES;
     uint4* recv = reinterpret_cast<uint4*>(vbuf + NV * C::V_BYTES);                 // [NZW][512 threads]
     float* recv_q = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(recv) + C::RECV_Z_BYTES);   // [512 threads]
@@ -189,15 +191,15 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
             mbar_init(smem_u32(&bars->v_full[s]), 1);
             mbar_init(smem_u32(&bars->v_empty[s]), 1);
         }
-        for (int s = 0; s < kNLP; ++s) {
-            mbar_init(smem_u32(&bars->l_free[s]), kEpiWarpsP);
+        for (int s = 0; s < kBufs; ++s) {
+            mbar_init(smem_u32(&bars->l_free[s]), kEpiWarpsP / 2);
         }
-        for (int s = 0; s < kNSP; ++s) {
-            mbar_init(smem_u32(&bars->s_written[s]), kEpiWarpsP);
+        for (int s = 0; s < kBufs; ++s) {
+            mbar_init(smem_u32(&bars->s_written[s]), kEpiWarpsP / 2);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kBufs; ++b) {
             mbar_init(smem_u32(&bars->dh_full[b]), 3);
-            mbar_init(smem_u32(&bars->a_ready[b]), 2 * kEpiWarpsP);
+            mbar_init(smem_u32(&bars->a_ready[b]), kEpiWarpsP);
             mbar_init(smem_u32(&bars->a_free[b]), 1);
         }
         mbar_init(smem_u32(&bars->z_full), 1);
@@ -240,7 +242,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     int err_layer = 0;
 
     // A pass q = -1 .. L-1 walks the nch chunks once.  Pass q >= 0 applies the update of layer q; pass q < L-1
-    // feeds the V contraction of layer q+1.  Chunk number n (all tiles, all passes) uses buffer n & 1.
+    // feeds the V contraction of layer q+1.  Chunk number n (all tiles, all passes) uses buffer n % 4.
     if (warp == 0) {
         // =============================== TMA producer: activations ==================
         {
@@ -255,7 +257,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
             while (nh < total_h && !err) {
                 err_layer = hq < 0 ? 0 : hq;
                 // The epilogue threads wait for one barrier per chunk (a look at an mbarrier costs them a few hundred
-                // cycles): the bytes of the old values are counted on the chunk's own barrier (slot n & 1 = buffer n & 1).
+                // cycles): the bytes of the old values are counted on the chunk's own barrier (slot n % 4 = buffer n % 4).
                 // pass >= 1 reads what this CTA stored one pass (nch chunks) earlier
                 if (hq >= 1) {
                     uint32_t idle = 0;
@@ -277,21 +279,19 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     if (hints) {
                         const uint64_t pol = hq >= 1 ? pol_h : pol_w;      // x is read once
                         tma_load_2d_hint(dst, src, col0 + hc * kCWP, m0, bar, pol);
-                        tma_load_2d_hint(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar, pol);
                     } else {
                         tma_load_2d(dst, src, col0 + hc * kCWP, m0, bar);
-                        tma_load_2d(dst + 16384, src, col0 + hc * kCWP + 64, m0, bar);
                     }
                 }
                 __syncwarp();
-                hp.step(kNLP);
+                hp.step(kBufs);
                 ++nh;
                 if (++hc == nch) { hc = 0; if (++hq == p.L) { hq = -1; ++ht; } }
             }
             // copies requested before giving up still land in shared memory: wait for them
             if (err || *abort_flag)
-                for (long long m = nh - 1; m >= 0 && m >= nh - kNLP; --m)
-                    mbar_wait(smem_u32(&bars->dh_full[m % kNLP]), uint32_t(m / kNLP) & 1u, kDrainPolls);
+                for (long long m = nh - 1; m >= 0 && m >= nh - kBufs; --m)
+                    mbar_wait(smem_u32(&bars->dh_full[m % kBufs]), uint32_t(m / kBufs) & 1u, kDrainPolls);
         }
     } else if (warp == kWarpU) {
         // =============================== TMA producer: U' ==========================
@@ -314,10 +314,10 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 #pragma unroll
                     for (int t = 0; t < C::UT; ++t)
                         if (hints)
-                            tma_load_2d_pair_hint(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
+                            tma_load_2d_pair_hint(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + (kCWP / 2) * hf,
                                                   ufull_lead + 8u * up.st, pol_w);
                         else
-                            tma_load_2d_pair(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + 64 * hf,
+                            tma_load_2d_pair(dst + t * C::U_TILE_BYTES, &tmU, 64 * t, uq * p.d + col0 + uc * kCWP + (kCWP / 2) * hf,
                                              ufull_lead + 8u * up.st);
                 }
                 __syncwarp();
@@ -349,14 +349,10 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     const uint32_t dst = vbuf_s + vp.st * C::V_BYTES;
                     DLP_T(2, vq - 1, vc, 0);
                     if (hf == 0) mbar_arrive_expect_tx(smem_u32(&bars->v_full[vp.st]), 2 * C::V_BYTES);
-#pragma unroll
-                    for (int t = 0; t < 2; ++t)
-                        if (hints)
-                            tma_load_2d_pair_hint(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
-                                                  vfull_lead + 8u * vp.st, pol_w);
-                        else
-                            tma_load_2d_pair(dst + t * C::V_TILE_BYTES, &tmV, col0 + vc * kCWP + 64 * t, vq * R + (R / 2) * hf,
-                                             vfull_lead + 8u * vp.st);
+                    if (hints)
+                        tma_load_2d_pair_hint(dst, &tmV, col0 + vc * kCWP, vq * R + (R / 2) * hf, vfull_lead + 8u * vp.st, pol_w);
+                    else
+                        tma_load_2d_pair(dst, &tmV, col0 + vc * kCWP, vq * R + (R / 2) * hf, vfull_lead + 8u * vp.st);
                 }
                 __syncwarp();
                 vp.step(NV);
@@ -378,11 +374,11 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
             uint32_t n = 0;
             uint32_t c_s = 0;
             for (int t = 0; t < my_tiles && !err; ++t) {
-                // the pass over x goes through the buffers too (chunk n: buffer n & 1): nothing to multiply, but the
+                // the pass over x goes through the buffers too (chunk n: buffer n % 4): nothing to multiply, but the
                 // chunk's barrier gets its commit (which arrives at once) when the buffer is free
                 for (int c = 0; c < nch && !err; ++c, ++n) {
-                    const uint32_t b = n & 1u;
-                    if (!wait_cta(smem_u32(&bars->a_free[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    const uint32_t b = n % kBufs;
+                    if (!wait_cta(smem_u32(&bars->a_free[b]), ((n / kBufs) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     if (elect_one()) umma_commit2_mask(smem_u32(&bars->dh_full[b]), pair_mask);
                     __syncwarp();
                 }
@@ -394,13 +390,13 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     ++c_s;
                     tc_fence_after();
                     for (int c = 0; c < nch; ++c, ++n) {
-                        const uint32_t b = n & 1u;
+                        const uint32_t b = n % kBufs;
                         // the weights land early: wait for them first, off the critical path
                         if (!wait_cluster(smem_u32(&bars->u_full[up.st]), up.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                         DLP_T(3, q, c, 1);
-                        const uint32_t acc = tmem_base + kBufCol + b * 128u;
-                        // the buffer is free once the V contraction of the chunk two before has read it
-                        if (!wait_cta(smem_u32(&bars->a_free[b]), ((n >> 1) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        const uint32_t acc = tmem_base + kBufCol + b * uint32_t(kCWP);
+                        // the buffer is free once the V contraction of the chunk four before has read it
+                        if (!wait_cta(smem_u32(&bars->a_free[b]), ((n / kBufs) & 1u) ^ 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         DLP_T(3, q, c, 2);
                         tc_fence_after();
                         const uint32_t ub = ubuf_s + up.st * C::U_BYTES;
@@ -425,7 +421,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         }
     } else if (warp == 2) {
         // =============================== V-MMA warp (leader) =======================
-        // z(q+1)[256 x R] += h_new[chunk][256 x 128] * V'[q+1][:, chunk]^T, A = the updated chunk in tensor memory
+        // z(q+1)[256 x R] += h_new[chunk][256 x 64] * V'[q+1][:, chunk]^T, A = the updated chunk in tensor memory
         if (hf == 0) {
             constexpr uint32_t idesc_v = umma_idesc_bf16(256, R);
             RingPos vp;
@@ -435,20 +431,20 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     err_layer = q;
                     const bool feeds = q + 1 < p.L;
                     for (int c = 0; c < nch; ++c, ++n) {
-                        const uint32_t b = n & 1u;
+                        const uint32_t b = n % kBufs;
                         // the weights land early: wait for them first, off the critical path
                         if (feeds && !wait_cluster(smem_u32(&bars->v_full[vp.st]), vp.ph)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                         DLP_T(4, q, c, 1);
-                        if (!wait_cluster(smem_u32(&bars->a_ready[b]), (n >> 1) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                        if (!wait_cluster(smem_u32(&bars->a_ready[b]), (n / kBufs) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                         DLP_T(4, q, c, 2);
                         tc_fence_after();
                         if (feeds) {
-                            const uint32_t a0 = tmem_base + kBufCol + b * 128u;
+                            const uint32_t a0 = tmem_base + kBufCol + b * uint32_t(kCWP);
                             const uint32_t vb = vbuf_s + vp.st * C::V_BYTES;
                             if (elect_one()) {
 #pragma unroll
                                 for (int k = 0; k < kCWP / 16; ++k) {
-                                    const uint64_t bdesc = umma_desc(vb + uint32_t(k / 4) * C::V_TILE_BYTES, 2u, 1024u) + uint64_t(2 * (k % 4));
+                                    const uint64_t bdesc = umma_desc(vb, 2u, 1024u) + uint64_t(2 * k);
                                     umma_ts2(tmem_base + kZCol, a0 + uint32_t(32 * (k / 2) + 8 * (k % 2)), bdesc, idesc_v, (c | k) ? 1u : 0u);
                                 }
                                 umma_commit2_mask(smem_u32(&bars->v_empty[vp.st]), pair_mask);
@@ -473,23 +469,22 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     } else if (warp == 3) {
         // =============================== store warp ================================
         // new chunk -> output buffer.  A slot is released when the copy has read it; the chunk counts as
-        // stored (readable by the next pass) once its bulk group is complete, which is checked two chunks late
+        // stored (readable by the next pass) once its bulk group is complete, which is checked four chunks late
         // so that this warp never waits for a write in flight.
         {
             RingPos sp;
             const uint64_t pol_h = l2_policy_evict_last(), pol_out = l2_policy_evict_first();
             const bool hints = !(PROF && (p.exp & 32));
             unsigned int n = 0;              // chunks seen (all tiles, all passes): the producer counts the same way
-            // the store slots of the first two chunks are free from the start
+            // the store slots of the first four chunks are free from the start
             if (lane == 0) {
-                mbar_arrive(smem_u32(&bars->dh_full[0]));
-                mbar_arrive(smem_u32(&bars->dh_full[1]));
+                for (int b = 0; b < kBufs; ++b) mbar_arrive(smem_u32(&bars->dh_full[b]));
             }
             __syncwarp();
             for (int t = 0; t < my_tiles && !err; ++t) {
                 const int m0 = (cl + t * ncl) * 2 * kRowsP + hf * kRowsP;
-                // (the pass over x stores nothing but walks the slots like the others: chunk n uses slot n & 1, as it
-                // uses buffer n & 1)
+                // (the pass over x stores nothing but walks the slots like the others: chunk n uses slot n % 4, as it
+                // uses buffer n % 4)
                 for (int q = -1; q < p.L && !err; ++q) {
                     err_layer = q;
                     for (int c = 0; c < nch; ++c, ++n) {
@@ -498,25 +493,21 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                             DLP_T(5, q, c, 0);
                             if (q >= 0 && m0 < p.M && !(PROF && (p.exp & 8))) {   // a CTA whose rows lie wholly past the batch stores nothing
                                 const uint32_t src = sbuf_s + sp.st * kHBytesP;
-                                if (hints) {       // the last layer's output is not read again here: first to leave L2
-                                    const uint64_t pol = q + 1 < p.L ? pol_h : pol_out;
-                                    tma_store_2d_hint(&tmY, col0 + c * kCWP, m0, src, pol);
-                                    tma_store_2d_hint(&tmY, col0 + c * kCWP + 64, m0, src + 16384, pol);
-                                } else {
-                                    tma_store_2d(&tmY, col0 + c * kCWP, m0, src);
-                                    tma_store_2d(&tmY, col0 + c * kCWP + 64, m0, src + 16384);
-                                }
+                                // (the last layer's output is not read again here: first to leave L2)
+                                if (hints) tma_store_2d_hint(&tmY, col0 + c * kCWP, m0, src, q + 1 < p.L ? pol_h : pol_out);
+                                else tma_store_2d(&tmY, col0 + c * kCWP, m0, src);
                             }
                             bulk_commit_group();
-                            bulk_wait_group_read<0>();
+                            // the slot of the chunk before has been read and is free for the chunk four after it: one of
+                            // the three arrivals that chunk's barrier waits for
+                            bulk_wait_group_read<1>();
                             DLP_T(5, q, c, 1);
-                            // the slot is free for the chunk after next: one of the three arrivals its barrier waits for
-                            mbar_arrive(smem_u32(&bars->dh_full[sp.st]));
-                            bulk_wait_group<2>();            // every group but the last two is complete
-                            if (n + 1u > *stored + 2u) *stored = n + 1u - 2u;
+                            if (n > 0) mbar_arrive(smem_u32(&bars->dh_full[(n - 1u) % kBufs]));
+                            bulk_wait_group<kStoreLag>();    // every group but the last ones is complete
+                            if (n + 1u > *stored + kStoreLag) *stored = n + 1u - kStoreLag;
                         }
                         __syncwarp();
-                        sp.step(kNSP);
+                        sp.step(kBufs);
                     }
                 }
             }
@@ -524,16 +515,17 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         }
     } else if (warp >= 4) {
         // =============================== epilogue warps =============================
-        // Four threads per row: thread (row er, quarter cq) owns 32 of the 128 columns of every chunk and a
-        // quarter of the columns of z.  Warp w reads tensor-memory lanes 32 * (w % 4) .. + 31.  Sixteen warps,
+        // Four threads per row: thread (row er, quarter cq) owns a quarter of the columns of z, and 32 (half hc) of the
+        // 64 columns of every chunk of parity g.  Warp w reads tensor-memory lanes 32 * (w % 4) .. + 31.  Sixteen warps,
         // four per scheduler: the per-chunk chain of one warp (wait, tensor-memory load, add, pack, store,
         // signal) is latency-bound, and the other three fill its gaps.
         const int q4 = warp & 3;
         const int cq = (warp - 4) >> 2;
+        const int g = cq >> 1, hc = cq & 1;
         const int er = 32 * q4 + lane;
         const int et = int(threadIdx.x) - 128;            // = cq * 128 + er
         const uint32_t tl = tmem_base + (uint32_t(32 * q4) << 16);
-        uint32_t n = 0;                      // chunks seen (all passes): phase of the A operand's barriers
+        uint32_t n = uint32_t(g);            // this group's next chunk (all passes; a pass has an even number)
         uint32_t c_z = 0;
         // barriers of the leader that this warp signals: its own if this CTA leads, else through the cluster window
         const uint32_t l_a_ready = hf ? mapa(smem_u32(&bars->a_ready[0]), lead) : smem_u32(&bars->a_ready[0]);
@@ -543,30 +535,29 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
             else mbar_arrive(bar);
         };
 
-        RingPos lp, sp;
         const int trole = (warp == 4 && lane == 0) ? 6 : ((warp == 19 && lane == 0) ? 7 : -1);
 #define DLP_TE(layer, chunk, event) do { if (PROF && trole >= 0) DLP_T(trole, layer, chunk, event); } while (0)
         const uint32_t x7 = uint32_t(er & 7);
-        // this thread's 64 bytes of its row inside a staging slot: tile cq / 2, 16-byte pieces 4 (cq % 2) .. + 3
-        const uint32_t row_off = uint32_t((cq >> 1) * 16384 + er * 128);
-        const uint32_t piece0 = uint32_t((cq & 1) * 4);
+        // this thread's 64 bytes of its row inside a staging slot: 16-byte pieces 4 hc .. + 3
+        const uint32_t row_off = uint32_t(er * 128);
+        const uint32_t piece0 = uint32_t(hc * 4);
         for (int t = 0; t < my_tiles && !err; ++t) {
             float ssq0 = 0.f, ssq1 = 0.f;
             for (int q = -1; q < p.L && !err; ++q) {
                 err_layer = q;
-                for (int c = 0; c < nch; ++c, ++n) {
-                    const uint32_t b = n & 1u;
-                    const uint32_t buf = tl + kBufCol + b * 128u + uint32_t(32 * cq);   // this thread's 32 columns of the buffer
+                for (int c = g; c < nch; c += 2, n += 2) {
+                    const uint32_t b = n % kBufs;
+                    const uint32_t buf = tl + kBufCol + b * uint32_t(kCWP) + uint32_t(32 * hc);   // this thread's 32 columns of the buffer
                     // ---- old values of the chunk: this thread's 64 bytes of its row, from the staging slot
                     DLP_TE(q, c, 0);
                     // ---- the one wait of a chunk: dh is in the buffer (in the pass over x: the buffer is free), the old
                     // values of the chunk have landed in their slot and the store slot is free
-                    if (!wait_cta(smem_u32(&bars->dh_full[b]), (n >> 1) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
+                    if (!wait_cta(smem_u32(&bars->dh_full[b]), (n / kBufs) & 1u)) { err = DLRB200_ERR_TIMEOUT_BARRIER; break; }
                     tc_fence_after();
                     DLP_TE(q, c, 1);
                     uint32_t cur[16];
                     {
-                        const uint8_t* rowp = lbuf + lp.st * kHBytesP + row_off;
+                        const uint8_t* rowp = lbuf + b * kHBytesP + row_off;
                         if (PROF && (p.exp & 1)) rowp = lbuf + lane * 16;     // experiment: no bank-spread reads
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
@@ -583,7 +574,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                         // the old values are in registers (the loads above have returned by now): the slot can take the
                         // next chunk
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&bars->l_free[lp.st]));
+                        if (lane == 0) mbar_arrive(smem_u32(&bars->l_free[b]));
                         DLP_TE(q, c, 3);
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
@@ -598,7 +589,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     } else {
                         // pass over x: the chunk goes to the tensor core as it is
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&bars->l_free[lp.st]));
+                        if (lane == 0) mbar_arrive(smem_u32(&bars->l_free[b]));
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
                             const float f0 = bf16lo_to_f(cur[j]), f1 = bf16hi_to_f(cur[j]);
@@ -606,7 +597,6 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                             ssq1 = fmaf(f1, f1, ssq1);
                         }
                     }
-                    lp.step(kNLP);
                     // ---- the chunk (bf16) becomes the A operand of the next layer's contraction, over this thread's own
                     // columns of dh: first, because the tensor core waits for it
                     DLP_TE(q, c, 4);
@@ -619,7 +609,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                     // ---- new values into a store slot: the store warp copies the slot out
                     {
                         if (q >= 0) {
-                            uint8_t* rowp = sbuf + sp.st * kHBytesP + row_off;
+                            uint8_t* rowp = sbuf + b * kHBytesP + row_off;
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
                                 if (!(PROF && (p.exp & 4))) *reinterpret_cast<uint4*>(rowp + (((piece0 + uint32_t(j)) ^ x7) << 4)) =
@@ -627,8 +617,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                             fence_async_smem();
                         }
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&bars->s_written[sp.st]));
-                        sp.step(kNSP);
+                        if (lane == 0) mbar_arrive(smem_u32(&bars->s_written[b]));
                     }
                     DLP_TE(q, c, 7);
                 }
@@ -748,13 +737,13 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 // of a layer, which grows with the exchange steps), where the clusters of a round are as many as can be resident
 // and no more than keep the rows in flight inside L2: every layer rewrites its tile in place, and once the tiles
 // of a round outgrow L2 each layer's traffic goes to DRAM (measured at d = 4096: 16384 rows at once 8.2 ms, in
-// two rounds of 8448 rows 6.6 ms).  Every pair keeps at least four chunks (the store warp reports a chunk as
-// stored two chunks late and the producer runs up to three chunks ahead).
+// two rounds of 8448 rows 6.6 ms).  Every pair keeps at least 512 columns, eight chunks: the store warp reports a chunk
+// as stored four chunks late, and the next pass's load of it is asked for up to four chunks ahead.
 struct PairShape { int pp, clusters; };
 PairShape pick_shape(int num_tiles, int d, int r, const int (&max_clusters)[3], size_t l2_bytes) {
     int forced = 0;
     if (const char* e = getenv("DLRB200_PAIR_SPLIT")) forced = atoi(e);
-    const int nch = d / kCWP;
+    const int nch = d / 128;                  // (in units of 128 columns)
     const double t_chunk = r == 128 ? 0.98 : 0.85;
     const size_t tile_bytes = size_t(2 * kRowsP) * d * 2;
     int fit = int(double(l2_bytes) * 0.62 / double(tile_bytes));      // tiles whose rows stay in L2 beside the weight stream
@@ -832,7 +821,7 @@ int launch_pair(void* enc, const void* x, void* y, const void* Vp, const void* U
         plan_only->path = DLRB200_PATH_STREAMED_PAIRS;
         plan_only->grid = grid;
         plan_only->cluster = 2 * pp;
-        plan_only->stripe_cols = kCWP;
+        plan_only->stripe_cols = 128;
         plan_only->rows_per_pass = 2 * kRowsP;
         plan_only->passes = (num_tiles + clusters - 1) / clusters;
         plan_only->stages = C::NU + C::NV;
@@ -843,7 +832,7 @@ int launch_pair(void* enc, const void* x, void* y, const void* Vp, const void* U
     if (!encode_2d_bf16(enc, &tmX, x, uint64_t(d), uint64_t(M), 64, kRowsP, 128) ||
         !encode_2d_bf16(enc, &tmY, y, uint64_t(d), uint64_t(M), 64, kRowsP, 128) ||
         !encode_2d_bf16(enc, &tmV, Vp, uint64_t(d), uint64_t(L) * R, 64, R / 2, 128) ||
-        !encode_2d_bf16(enc, &tmU, Up, uint64_t(R), uint64_t(L) * d, 64, 64, 128))
+        !encode_2d_bf16(enc, &tmU, Up, uint64_t(R), uint64_t(L) * d, 64, kCWP / 2, 128))
         return DLRB200_ERR_CUDA;
     PParams p;
     p.M = M; p.d = d; p.L = L;
@@ -877,7 +866,7 @@ int dispatch_pair(void* enc, const void* x, void* y, const void* Vp, const void*
 
 }  // namespace
 
-bool stream_pair_supported(int d, int r) { return (r == 64 || r == 128) && d % kCWP == 0 && d >= 4 * kCWP; }
+bool stream_pair_supported(int d, int r) { return (r == 64 || r == 128) && d % 128 == 0 && d >= 512; }
 
 int stream_pair_plan(int M, int d, int r, int L, int num_sms, int smem_optin, dlrb200_plan* plan) {
     const size_t ws = plan->workspace_bytes;

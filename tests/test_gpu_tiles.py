@@ -49,3 +49,11 @@ def test_cluster_kernel(d, r, L, M, stripe, monkeypatch):
     monkeypatch.setenv("DLRB200_CLUSTER_STRIPE", str(stripe))
     assert D.ops.query_call(M, d, r, L).stripe_cols == (512 if d > 2048 else stripe)
     _check(d, r, L, M, 2)
+
+
+# the pair kernel: the fewest chunks a pair can have (eight), one, two and four pairs per cluster, one layer, several tiles
+@pytest.mark.parametrize("d,r,L,M", [(512, 64, 1, 65), (512, 128, 3, 257), (640, 128, 2, 300), (1024, 64, 2, 130), (2048, 128, 2, 513),
+                                     (4096, 128, 1, 300), (512, 64, 2, 74 * 256 + 1), (512, 128, 3, 150 * 256 + 70)])
+def test_pair_kernel(d, r, L, M, monkeypatch):
+    monkeypatch.setenv("DLRB200_FORCE_PATH", "5")
+    _check(d, r, L, M, 5)
