@@ -337,7 +337,10 @@ bool use_resident(int M, int d, int r, int L, const DevInfo& di, dlrb200_plan* p
     if (forced != 0 || M <= 64) return true;
     double other = 1e30;
     large_batch_path(M, d, r, L, di, &other);
-    return us < 0.75 * other;             // (near a tie the large-batch kernel, whose time does not grow with the rows)
+    // (near a tie the large-batch kernel, whose time does not grow with the rows.  Measured, resident / cluster, us: d = 2048,
+    // 333 rows 381 / 552, 500 rows 673 / 555; d = 1024, 600 rows 275 / 450, 1100 rows 489 / 450; d = 4096, 200 rows 652 / 1068,
+    // 300 rows 1171 / 1078)
+    return us < 0.9 * other;
 }
 
 bool use_stream_path(int M, int d, int r, int L, const DevInfo& di) {
