@@ -69,7 +69,7 @@ class DLRNet(nn.Module):
         self.rms_w = nn.ParameterList([nn.Parameter(torch.ones(d)) for _ in range(depth)])
         self.alphas = nn.ParameterList([nn.Parameter(torch.tensor(float(alpha_init))) for _ in range(depth)])
         self.use_checkpoint = True
-        self._folded = None       # (key, V', U') derived cache, rebuilt when parameters change
+        self._folded = None       # (key, V', U', parameters) derived cache, rebuilt when parameters change
         self.fast = True          # set False to force the torch loop
 
     # ---- adoption of an existing (reference) module's parameters -------------
@@ -89,9 +89,11 @@ class DLRNet(nn.Module):
 
     # ---- derived folded weights ----------------------------------------------
     def _param_dicts(self):
-        """The parameters as four dicts (V, U, gains, alphas), layer by layer."""
-        return tuple(p._parameters if isinstance(p, nn.ParameterList) else {str(i): t for i, t in enumerate(p)}
-                     for p in (self.Vs, self.Us, self.rms_w, self.alphas))
+        """The parameters as four dicts (V, U, gains, alphas), in the order of the layers: a list's own dict where it holds
+        exactly that, else (an entry is pruned or parametrized, or was set again) what indexing the list gives."""
+        in_order = _lib.host().in_order
+        return tuple(p._parameters if isinstance(p, nn.ParameterList) and in_order(p._parameters, len(p))
+                     else {str(i): t for i, t in enumerate(p)} for p in (self.Vs, self.Us, self.rms_w, self.alphas))
 
     def _cache_key(self):
         # every parameter of every layer: storage address and in-place version counter.  A write through
@@ -105,7 +107,12 @@ class DLRNet(nn.Module):
 
     def folded_weights(self):
         """(V' (L,r,d), U' (L,d,r)) bf16 on the parameters' device, cached."""
-        dicts, host = self._param_dicts(), _lib.host()
+        host = _lib.host()
+        if self._folded is not None:
+            own = tuple(getattr(p, "_parameters", None) for p in (self.Vs, self.Us, self.rms_w, self.alphas))
+            if host.unchanged(self._folded[0], own):           # (no, for dicts that do not hold the lists' entries in order)
+                return self._folded[1], self._folded[2]
+        dicts = self._param_dicts()
         if self._folded is None or not host.unchanged(self._folded[0], dicts):
             found = host.layers(dicts)
             if found is not None:
@@ -113,7 +120,8 @@ class DLRNet(nn.Module):
             else:
                 V, U, w, a = (torch.stack([p.detach() for p in d.values()]) for d in dicts)
                 Vp, Up = ops.fold_weights(V, U, w, a)
-            self._folded = (host.snapshot(dicts), Vp, Up)
+            # (with the dicts: a tensor computed on access must outlive its address in the key)
+            self._folded = (host.snapshot(dicts), Vp, Up, dicts)
         return self._folded[1], self._folded[2]
 
     def _load_from_state_dict(self, *args, **kwargs):

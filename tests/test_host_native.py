@@ -1,6 +1,8 @@
 """The native walk over a net's parameters (csrc/host.cpp)."""
+import pytest
 import torch
 import torch.nn as nn
+from torch.nn.utils import parametrize, prune
 
 import dlr_lock_b200 as D
 from dlr_lock_b200.build import build_library
@@ -27,3 +29,52 @@ def test_any_change_of_a_parameter_is_seen():
     assert not host.unchanged(key, dicts()) and host.unchanged(host.snapshot(dicts()), dicts())
     # parameters on the CPU are not for the fold kernel
     assert host.layers(dicts()) is None and host.state_layers(net.state_dict()) is None
+
+
+class _Scaled(nn.Module):
+    def forward(self, w):
+        return 0.5 * w
+
+
+def _pruned(net):
+    prune.l1_unstructured(net.Vs, "0", 0.5)
+
+
+def _prune_removed(net):                                       # a plain parameter again, but last in the list's own dict
+    prune.l1_unstructured(net.Vs, "0", 0.5)
+    prune.remove(net.Vs, "0")
+
+
+def _parametrized_one(net):
+    parametrize.register_parametrization(net.Vs, "0", _Scaled())
+
+
+def _parametrized_all(net):
+    for p in (net.Vs, net.Us, net.rms_w, net.alphas):
+        parametrize.register_parametrization(p, "1", _Scaled())
+
+
+@pytest.mark.parametrize("change", [None, _pruned, _prune_removed, _parametrized_one, _parametrized_all])
+def test_layers_are_folded_as_the_lists_give_them(change, monkeypatch):
+    build_library()
+    monkeypatch.setattr(D.ops, "fold_weights", lambda V, U, w, a: (V * w[:, None, :], a[:, None, None] * U))
+    torch.manual_seed(0)
+    net = D.DLRNet(32, 4, 3, alpha_init=0.7)
+    with torch.no_grad():
+        for i in range(3):
+            net.rms_w[i].normal_(1.0, 0.1)
+    if change is not None:
+        change(net)
+
+    def check():
+        Vp, Up = net.folded_weights()
+        for i in range(3):
+            assert torch.equal(Vp[i], net.Vs[i] * net.rms_w[i]) and torch.equal(Up[i], net.alphas[i] * net.Us[i]), i
+
+    with torch.no_grad():
+        check()
+        if change in (None, _pruned, _prune_removed):
+            assert net.folded_weights()[0] is net.folded_weights()[0]          # nothing changed: not folded again
+        # an edit below a parametrization moves a tensor that is computed on each access
+        getattr(net.Vs.parametrizations, "0").original.mul_(2.0) if change is _parametrized_one else net.Vs[0].mul_(2.0)
+        check()
