@@ -10,7 +10,8 @@
 //
 // The last two return (L, r, d, device index, matrices are bf16, alphas are bf16, addresses of V, U, gain, alpha as four
 // bytes objects), or None for anything but complete layers of contiguous bf16 or fp32 tensors of one shape on one GPU; the
-// caller then takes the general way through torch operations.
+// caller then takes the general way through torch operations.  A C++ exception becomes a Python one: the address of a tensor
+// without storage (under a functorch transform) is a RuntimeError, as it is for Tensor.data_ptr().
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -18,6 +19,7 @@
 #include <string>
 #include <vector>
 
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 namespace {
@@ -29,7 +31,7 @@ struct Word {
 Word word_of(PyObject* o) {
     const at::Tensor& t = THPVariable_Unpack(o);
     const auto& vc = t.unsafeGetTensorImpl()->version_counter();
-    return Word{reinterpret_cast<uint64_t>(t.has_storage() ? t.const_data_ptr() : nullptr), vc.enabled() ? vc.current_version() : 0};
+    return Word{reinterpret_cast<uint64_t>(t.const_data_ptr()), vc.enabled() ? vc.current_version() : 0};
 }
 
 // "0", "1", ... as text, and whether a key is the one that is due.
@@ -69,6 +71,7 @@ bool for_each_tensor(PyObject* dicts, F f) {
 }
 
 PyObject* snapshot(PyObject*, PyObject* dicts) {
+    HANDLE_TH_ERRORS
     if (!PyTuple_Check(dicts)) {
         PyErr_SetString(PyExc_TypeError, "snapshot takes a tuple of dicts of tensors, keys \"0\", \"1\", ... in order");
         return nullptr;
@@ -79,9 +82,11 @@ PyObject* snapshot(PyObject*, PyObject* dicts) {
         return nullptr;
     }
     return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(words.data()), Py_ssize_t(words.size() * sizeof(Word)));
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* unchanged(PyObject*, PyObject* args) {
+    HANDLE_TH_ERRORS
     PyObject *snap, *dicts;
     if (!PyArg_ParseTuple(args, "O!O!", &PyBytes_Type, &snap, &PyTuple_Type, &dicts)) return nullptr;
     const char* at = PyBytes_AS_STRING(snap);
@@ -93,6 +98,7 @@ PyObject* unchanged(PyObject*, PyObject* args) {
         return true;
     });
     return PyBool_FromLong(same && at == end);
+    END_HANDLE_TH_ERRORS
 }
 
 struct Group {
@@ -119,6 +125,7 @@ long number(const char* s) {
 }
 
 PyObject* in_order(PyObject*, PyObject* args) {
+    HANDLE_TH_ERRORS
     PyObject* d;
     Py_ssize_t n;
     if (!PyArg_ParseTuple(args, "O!n", &PyDict_Type, &d, &n)) return nullptr;
@@ -128,6 +135,7 @@ PyObject* in_order(PyObject*, PyObject* args) {
     bool same = PyDict_GET_SIZE(d) == n;
     while (same && PyDict_Next(d, &pos, &key, &value)) same = count.is(key);
     return PyBool_FromLong(same);
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* describe(const Group (&g)[4]) {
@@ -143,6 +151,7 @@ PyObject* describe(const Group (&g)[4]) {
         for (size_t i = 0; i < L; ++i) {
             if (!g[k].at[i]) Py_RETURN_NONE;
             const at::Tensor& t = THPVariable_Unpack(g[k].at[i]);
+            if (!t.has_storage()) Py_RETURN_NONE;
             if (k == 0 && i == 0) {
                 if (t.dim() != 2 || !t.is_cuda()) Py_RETURN_NONE;
                 r = t.size(0);
@@ -160,7 +169,9 @@ PyObject* describe(const Group (&g)[4]) {
                               : k == 2 ? t.dim() == 1 && t.size(0) == d
                                        : t.numel() == 1;
             if (!shaped) Py_RETURN_NONE;
-            address[k].push_back(reinterpret_cast<uint64_t>(t.const_data_ptr()));
+            const void* data = t.const_data_ptr();
+            if (!data) Py_RETURN_NONE;                 // (a fake tensor)
+            address[k].push_back(reinterpret_cast<uint64_t>(data));
         }
     }
     auto bytes = [&](int k) {
@@ -171,6 +182,7 @@ PyObject* describe(const Group (&g)[4]) {
 }
 
 PyObject* layers(PyObject*, PyObject* dicts) {
+    HANDLE_TH_ERRORS
     if (!PyTuple_Check(dicts) || PyTuple_GET_SIZE(dicts) != 4) {
         PyErr_SetString(PyExc_TypeError, "layers takes a tuple of four dicts");
         return nullptr;
@@ -191,9 +203,11 @@ PyObject* layers(PyObject*, PyObject* dicts) {
         }
     }
     return describe(g);
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* state_layers(PyObject*, PyObject* sd) {
+    HANDLE_TH_ERRORS
     if (!PyDict_Check(sd)) Py_RETURN_NONE;
     static const struct { const char* name; size_t n; } kNames[4] = {{"Vs.", 3}, {"Us.", 3}, {"rms_w.", 6}, {"alphas.", 7}};
     Group g[4];
@@ -213,6 +227,7 @@ PyObject* state_layers(PyObject*, PyObject* sd) {
             }
     }
     return describe(g);
+    END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef kMethods[] = {{"in_order", in_order, METH_VARARGS, nullptr},

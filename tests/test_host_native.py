@@ -2,6 +2,7 @@
 import pytest
 import torch
 import torch.nn as nn
+from torch._subclasses.fake_tensor import FakeTensorMode
 from torch.nn.utils import parametrize, prune
 
 import dlr_lock_b200 as D
@@ -78,3 +79,25 @@ def test_layers_are_folded_as_the_lists_give_them(change, monkeypatch):
         # an edit below a parametrization moves a tensor that is computed on each access
         getattr(net.Vs.parametrizations, "0").original.mul_(2.0) if change is _parametrized_one else net.Vs[0].mul_(2.0)
         check()
+
+
+def test_tensors_without_memory_of_their_own_raise_or_are_left_to_torch():
+    build_library()
+    host = D._lib.host()
+    one = lambda v: tuple({"0": t} for t in (v, v.detach().mT.contiguous(), torch.ones(32), torch.ones(())))
+
+    def layer(v):                                              # a batch of layers, of which none has an address
+        assert host.layers(one(v)) is None
+        for call in (host.snapshot, lambda dicts: host.unchanged(b"", dicts)):
+            with pytest.raises(RuntimeError):
+                call(one(v))
+        return v.sum()
+
+    V = torch.randn(2, 4, 32)
+    torch.vmap(layer)(V)
+    torch.func.grad(layer)(V[0])
+    with FakeTensorMode():
+        fake = [torch.empty(s, device="cuda", dtype=torch.bfloat16) for s in ((4, 32), (32, 4), (32,), ())]
+        assert host.layers(tuple({"0": t} for t in fake)) is None
+        assert host.state_layers(dict(zip(("Vs.0", "Us.0", "rms_w.0", "alphas.0"), fake))) is None
+        torch.vmap(lambda v: (host.layers(({"0": v},) + tuple({"0": t} for t in fake[1:])), v)[1])(torch.stack([fake[0]] * 2))
