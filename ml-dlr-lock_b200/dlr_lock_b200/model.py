@@ -93,7 +93,7 @@ class DLRNet(nn.Module):
         exactly that, else (an entry is pruned or parametrized, or was set again) what indexing the list gives."""
         in_order = _lib.host().in_order
         return tuple(p._parameters if isinstance(p, nn.ParameterList) and in_order(p._parameters, len(p))
-                     else {str(i): t for i, t in enumerate(p)} for p in (self.Vs, self.Us, self.rms_w, self.alphas))
+                     else {str(i): t.detach() for i, t in enumerate(p)} for p in (self.Vs, self.Us, self.rms_w, self.alphas))
 
     def _cache_key(self):
         # every parameter of every layer: storage address and in-place version counter.  A write through
@@ -118,7 +118,7 @@ class DLRNet(nn.Module):
             if found is not None:
                 Vp, Up = ops.fold_layers(found, round_alpha=False)
             else:
-                V, U, w, a = (torch.stack([p.detach() for p in d.values()]) for d in dicts)
+                V, U, w, a = (torch.stack([t.detach() for t in d.values()]) for d in dicts)
                 Vp, Up = ops.fold_weights(V, U, w, a)
             # (with the dicts: a tensor computed on access must outlive its address in the key)
             self._folded = (host.snapshot(dicts), Vp, Up, dicts)

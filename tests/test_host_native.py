@@ -1,4 +1,6 @@
 """The native walk over a net's parameters (csrc/host.cpp)."""
+import copy
+
 import pytest
 import torch
 import torch.nn as nn
@@ -79,6 +81,9 @@ def test_layers_are_folded_as_the_lists_give_them(change, monkeypatch):
         # an edit below a parametrization moves a tensor that is computed on each access
         getattr(net.Vs.parametrizations, "0").original.mul_(2.0) if change is _parametrized_one else net.Vs[0].mul_(2.0)
         check()
+    if change in (None, _parametrized_one, _parametrized_all):
+        net.folded_weights()                                   # with gradients on: the module can still be copied
+        copy.deepcopy(net).folded_weights()
 
 
 def test_tensors_without_memory_of_their_own_raise_or_are_left_to_torch():
