@@ -28,10 +28,10 @@ struct Word {
     uint64_t address, version;
 };
 
+// (raises for an inference tensor, whose edits leave no trace)
 Word word_of(PyObject* o) {
     const at::Tensor& t = THPVariable_Unpack(o);
-    const auto& vc = t.unsafeGetTensorImpl()->version_counter();
-    return Word{reinterpret_cast<uint64_t>(t.const_data_ptr()), vc.enabled() ? vc.current_version() : 0};
+    return Word{reinterpret_cast<uint64_t>(t.const_data_ptr()), t.unsafeGetTensorImpl()->version_counter().current_version()};
 }
 
 // "0", "1", ... as text, and whether a key is the one that is due.

@@ -114,6 +114,7 @@ class DLRNet(nn.Module):
                 return self._folded[1], self._folded[2]
         dicts = self._param_dicts()
         if self._folded is None or not host.unchanged(self._folded[0], dicts):
+            key = host.snapshot(dicts)
             found = host.layers(dicts)
             if found is not None:
                 Vp, Up = ops.fold_layers(found, round_alpha=False)
@@ -121,7 +122,7 @@ class DLRNet(nn.Module):
                 V, U, w, a = (torch.stack([t.detach() for t in d.values()]) for d in dicts)
                 Vp, Up = ops.fold_weights(V, U, w, a)
             # (with the dicts: a tensor computed on access must outlive its address in the key)
-            self._folded = (host.snapshot(dicts), Vp, Up, dicts)
+            self._folded = (key, Vp, Up, dicts)
         return self._folded[1], self._folded[2]
 
     def _load_from_state_dict(self, *args, **kwargs):

@@ -106,3 +106,14 @@ def test_tensors_without_memory_of_their_own_raise_or_are_left_to_torch():
         assert host.layers(tuple({"0": t} for t in fake)) is None
         assert host.state_layers(dict(zip(("Vs.0", "Us.0", "rms_w.0", "alphas.0"), fake))) is None
         torch.vmap(lambda v: (host.layers(({"0": v},) + tuple({"0": t} for t in fake[1:])), v)[1])(torch.stack([fake[0]] * 2))
+
+
+def test_parameters_whose_edits_are_not_counted_are_refused():
+    build_library()
+    with torch.inference_mode():
+        net = D.DLRNet(32, 4, 3)
+        with pytest.raises(RuntimeError, match="version counter"):
+            net.folded_weights()
+        key = b"\0" * (16 * 12)
+        with pytest.raises(RuntimeError, match="version counter"):
+            D._lib.host().unchanged(key, net._param_dicts())
