@@ -4,7 +4,8 @@
 //
 //   in_order(dict, n)        whether the keys of a dict are "0", "1", ... "n-1", in this order
 //   snapshot(dicts)          bytes: storage address and in-place version of every tensor of the dicts, in order
-//   unchanged(bytes, dicts)  whether snapshot(dicts) would return the same bytes (no, if it would refuse the dicts)
+//   unchanged(bytes, dicts)  whether snapshot(dicts) would return the same bytes (no, if it would refuse the dicts, and for
+//                            anything but bytes)
 //   layers(dicts)            what the fold kernel needs of the four parameter dicts (V, U, gains, alphas; keys "0", "1", ...)
 //   state_layers(dict)       the same of a state dict (keys Vs.i, Us.i, rms_w.i, alphas.i, an _orig_mod. prefix allowed)
 //
@@ -88,7 +89,8 @@ PyObject* snapshot(PyObject*, PyObject* dicts) {
 PyObject* unchanged(PyObject*, PyObject* args) {
     HANDLE_TH_ERRORS
     PyObject *snap, *dicts;
-    if (!PyArg_ParseTuple(args, "O!O!", &PyBytes_Type, &snap, &PyTuple_Type, &dicts)) return nullptr;
+    if (!PyArg_ParseTuple(args, "OO!", &snap, &PyTuple_Type, &dicts)) return nullptr;
+    if (!PyBytes_Check(snap)) Py_RETURN_FALSE;
     const char* at = PyBytes_AS_STRING(snap);
     const char* end = at + PyBytes_GET_SIZE(snap);
     const bool same = for_each_tensor(dicts, [&](PyObject* o) {

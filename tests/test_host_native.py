@@ -117,3 +117,13 @@ def test_parameters_whose_edits_are_not_counted_are_refused():
         key = b"\0" * (16 * 12)
         with pytest.raises(RuntimeError, match="version counter"):
             D._lib.host().unchanged(key, net._param_dicts())
+
+
+def test_a_key_of_another_kind_counts_as_changed(monkeypatch):
+    # a module that was saved whole, by a version whose key was a tuple
+    build_library()
+    monkeypatch.setattr(D.ops, "fold_weights", lambda V, U, w, a: (V * w[:, None, :], a[:, None, None] * U))
+    net = D.DLRNet(32, 4, 3)
+    net._folded = (tuple(range(24)), None, None)
+    Vp, Up = net.folded_weights()
+    assert torch.equal(Vp[2], net.Vs[2] * net.rms_w[2])
