@@ -81,15 +81,22 @@ def load() -> ctypes.CDLL:
 _host_module = None
 
 
+def host_path() -> str:
+    """Where the host helper for this Python and this torch lies: it is compiled against their C++ interfaces."""
+    import sys
+
+    import torch
+
+    return os.path.join(HERE, f"_host.{sys.implementation.cache_tag}-torch-{torch.__version__}.so")
+
+
 def host():
     """The native host helper ``_host`` (csrc/host.cpp), loaded once."""
     global _host_module
     if _host_module is None:
         import importlib.util
 
-        import torch  # noqa: F401  (its libraries, which the helper links against)
-
-        path = os.path.join(HERE, "_host.so")
+        path = host_path()
         if not os.path.exists(path):
             raise RuntimeError(f"{path} is missing: build it with `python -m dlr_lock_b200.build`.")
         spec = importlib.util.spec_from_file_location("_host", path)

@@ -17,12 +17,13 @@ import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
 
+from . import _lib
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.normpath(os.path.join(HERE, "..", "csrc"))
 INCLUDE = os.path.normpath(os.path.join(HERE, "..", "..", "include"))
 LIB_PATH = os.path.join(HERE, "libdlr_b200.so")
 HOST_SRC = os.path.join(CSRC, "host.cpp")
-HOST_PATH = os.path.join(HERE, "_host.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 NVCC_FLAGS = [
@@ -51,9 +52,11 @@ def _stale(target: str, deps) -> bool:
 
 
 def build_host(force: bool = False) -> str:
-    """Compile the host-side helper module ``_host`` against torch's headers, if it is out of date."""
-    if not force and not _stale(HOST_PATH, [HOST_SRC]):
-        return HOST_PATH
+    """Compile the host-side helper module ``_host`` against torch's headers, if there is none for this Python and torch or
+    its source is newer."""
+    path = _lib.host_path()
+    if not force and not _stale(path, [HOST_SRC]):
+        return path
     import sysconfig
 
     import torch
@@ -63,13 +66,13 @@ def build_host(force: bool = False) -> str:
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", sysconfig.get_paths()["include"]]
     for p in include_paths():
         cmd += ["-isystem", p]
-    cmd += [HOST_SRC, "-o", HOST_PATH]
+    cmd += [HOST_SRC, "-o", path]
     for p in library_paths():
         cmd += ["-L", p]
     r = subprocess.run(cmd + ["-ltorch_python", "-ltorch_cpu", "-lc10"], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
-    return HOST_PATH
+    return path
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:

@@ -127,3 +127,11 @@ def test_a_key_of_another_kind_counts_as_changed(monkeypatch):
     net._folded = (tuple(range(24)), None, None)
     Vp, Up = net.folded_weights()
     assert torch.equal(Vp[2], net.Vs[2] * net.rms_w[2])
+
+
+def test_a_helper_built_against_another_torch_is_not_loaded(monkeypatch):
+    build_library()
+    monkeypatch.setattr(D._lib, "_host_module", None)
+    monkeypatch.setattr(torch, "__version__", "0.0")
+    with pytest.raises(RuntimeError, match="build"):
+        D._lib.host()
