@@ -224,8 +224,7 @@ PyObject* state_layers(PyObject*, PyObject* sd) {
         if (std::strncmp(s, "_orig_mod.", 10) == 0) s += 10;
         for (int k = 0; k < 4; ++k)
             if (std::strncmp(s, kNames[k].name, kNames[k].n) == 0) {
-                const long i = number(s + kNames[k].n);
-                if (i >= 0 && !g[k].put(i, value)) Py_RETURN_NONE;
+                if (!g[k].put(number(s + kNames[k].n), value)) Py_RETURN_NONE;      // (no layer number either)
             }
     }
     return describe(g);

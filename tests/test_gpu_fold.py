@@ -38,3 +38,13 @@ def test_unaligned_and_unusual_parameters_take_the_general_way():
     mixed = D.pack_state_dict(dict(sd, **{"Us.2": sd["Us.2"].t().contiguous().t()}), "cuda")     # not contiguous
     for p in (got, mixed):
         assert torch.equal(p.Vp, want.Vp) and torch.equal(p.Up, want.Up)
+
+
+def test_what_is_not_a_net_is_refused():
+    import dlr_lock_b200 as D
+    torch.manual_seed(0)
+    sd = {k: v.to(torch.bfloat16).cuda() for k, v in D.DLRNet(64, 8, 3).state_dict().items()}
+    D.pack_state_dict(dict(sd, **{"Vs.extra": sd["Vs.0"]}), "cuda")             # (not a layer's name)
+    for key in ("Vs.3", "Vs.70000", "_orig_mod.alphas.4"):
+        with pytest.raises(ValueError):
+            D.pack_state_dict(dict(sd, **{key: sd["Vs.0"]}), "cuda")
