@@ -322,27 +322,6 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di, double* esti
     return path;
 }
 
-// Calls that the resident-cluster kernel serves instead of the kernel planned above, where it covers the shape: batches of
-// up to 64 rows (measured against the best of the others, us: d = 1024 110 / 281 at one row, 112 / 295 at 64; d = 2048
-// 151 / 332 at 8, 162 / 767 at 64; d = 4096 224 / 323 at one row, 237 / 524 at 16, 360 / 1093 at 64; at d = 5120 each of its
-// 16 CTAs pulls 328 KB a layer and the striped kernel's 80 are faster up to a dozen rows: 674 / 445 at one row, 648 / 828 at
-// 12), and beyond that wherever waves of small row groups end before the large-batch kernel's one pass over a tile: both
-// sides estimated from measured times.
-bool use_resident(int M, int d, int r, int L, const DevInfo& di, dlrb200_plan* plan = nullptr) {
-    const int forced = env_int("DLRB200_FORCE_PATH", 0);
-    if (!dlr::resident_supported(d, r) || (forced != 0 && forced != DLRB200_PATH_RESIDENT)) return false;
-    if (forced == 0 && M <= 64 && r >= 256 && M < 12) return false;
-    const double us = dlr::resident_estimate_us(M, d, r, L, di.smem_optin, plan);
-    if (us >= 1e30) return false;
-    if (forced != 0 || M <= 64) return true;
-    double other = 1e30;
-    large_batch_path(M, d, r, L, di, &other);
-    // (near a tie the large-batch kernel, whose time does not grow with the rows.  Measured, resident / cluster, us: d = 2048,
-    // 333 rows 381 / 552, 500 rows 673 / 555; d = 1024, 600 rows 275 / 450, 1100 rows 489 / 450; d = 4096, 200 rows 652 / 1068,
-    // 300 rows 1171 / 1078)
-    return us < 0.9 * other;
-}
-
 bool use_stream_path(int M, int d, int r, int L, const DevInfo& di) {
     return large_batch_path(M, d, r, L, di) == DLRB200_PATH_STREAMED;
 }
@@ -384,6 +363,33 @@ bool use_cluster_small(int M, int d, int r) {
     return (d <= 1024 && M >= 2) || (d <= 2048 && M > 16);
 }
 
+// The fewest rows of the striped kernel with the two-level exchange (below).
+int striped_clusters_from(int d, int r) { return d >= 4096 ? (r >= 256 ? 16 : 17) : (d >= 2048 ? 29 : 65); }
+
+// Calls that the resident-cluster kernel serves instead of the kernel planned above, where it covers the shape: batches of
+// up to 64 rows (measured against the best of the others, us: d = 1024 110 / 281 at one row, 118 / 295 at 64; d = 2048
+// 151 / 332 at 8, 162 / 767 at 64; d = 4096 224 / 323 at one row, 237 / 524 at 16, 360 / 1093 at 64; at d = 5120 each of its
+// 16 CTAs pulls 328 KB a layer and the striped kernel's 80 are faster up to a dozen rows: 674 / 445 at one row, 648 / 828 at
+// 12), and beyond that wherever waves of small row groups end before the large-batch kernel's one pass over a tile: both
+// sides estimated from measured times.
+// `terms`: the calls that the cluster-small kernel would serve, all in fp32, run on the form whose matrix operands are three
+// bf16 terms.
+bool use_resident(int M, int d, int r, int L, const DevInfo& di, bool* terms, dlrb200_plan* plan = nullptr) {
+    const int forced = env_int("DLRB200_FORCE_PATH", 0);
+    if (!dlr::resident_supported(d, r) || (forced != 0 && forced != DLRB200_PATH_RESIDENT)) return false;
+    if (forced == 0 && M <= 64 && r >= 256 && M < 12) return false;
+    *terms = use_cluster_small(M, d, r) && M < striped_clusters_from(d, r);
+    const double us = dlr::resident_estimate_us(M, d, r, L, *terms, di.smem_optin, plan);
+    if (us >= 1e30) return false;
+    if (forced != 0 || M <= 64) return true;
+    double other = 1e30;
+    large_batch_path(M, d, r, L, di, &other);
+    // (near a tie the large-batch kernel, whose time does not grow with the rows.  Measured, resident / cluster, us: d = 2048,
+    // 333 rows 381 / 552, 500 rows 673 / 555; d = 1024, 600 rows 275 / 450, 1100 rows 489 / 450; d = 4096, 200 rows 652 / 1068,
+    // 300 rows 1171 / 1078)
+    return us < 0.9 * other;
+}
+
 // Small batches on the striped kernel with the two-level exchange (decode_tl.cu).  Measured on a B200, L about
 // 143, against the best of the other small-batch kernels (us): d = 4096, r = 128: 665 against 719 at 17 rows,
 // 754 / 853 at 32, 1012 / 1177 at 48, 1109 / 1184 at 64 (there the other is one padded 128-row tile on one
@@ -396,10 +402,7 @@ bool use_striped_clusters(int M, int d, int r, int L, const DevInfo& di) {
     const int forced = env_int("DLRB200_FORCE_PATH", 0);
     if (M > 64) return false;
     if (forced != 0 && forced != DLRB200_PATH_STRIPED_CLUSTERS) return false;
-    if (forced == 0) {
-        const int from = d >= 4096 ? (r >= 256 ? 16 : 17) : (d >= 2048 ? 29 : 65);
-        if (M < from) return false;
-    }
+    if (forced == 0 && M < striped_clusters_from(d, r)) return false;
     dlrb200_plan pl;
     std::memset(&pl, 0, sizeof(pl));
     return striped_tl_launch(nullptr, nullptr, nullptr, nullptr, M, d, r, L, 0.f, nullptr, nullptr, nullptr, di, &pl) == DLRB200_OK;
@@ -511,7 +514,8 @@ int dlrb200_query_call(int M, int d, int r, int L, dlrb200_plan* plan) {
     DevInfo di;
     if (device_info(&di) != DLRB200_OK) return DLRB200_ERR_CUDA;
     dlrb200_plan resident = *plan;
-    if (use_resident(M, d, r, L, di, &resident)) *plan = resident;
+    bool terms = false;
+    if (use_resident(M, d, r, L, di, &terms, &resident)) *plan = resident;
     else if (plan->path == DLRB200_PATH_CLUSTER) return dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, plan, nullptr, false);
     return DLRB200_OK;
 }
@@ -531,11 +535,12 @@ int dlrb200_forward(const void* x, void* y, const void* Vp, const void* Up, int 
     if (rc != DLRB200_OK) return rc;
     if (di.cc_major != 10) return DLRB200_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (use_resident(M, d, r, L, di)) {
+    bool terms = false;
+    if (use_resident(M, d, r, L, di, &terms)) {
         EncodeTiledFn enc = encode_fn();
         if (!enc) return DLRB200_ERR_CUDA;
-        rc = dlr::resident_forward(reinterpret_cast<void*>(enc), x, y, Vp, Up, M, d, r, L, eps, status_dev, st, di.smem_optin,
-                                   spin_limit());
+        rc = dlr::resident_forward(reinterpret_cast<void*>(enc), x, y, Vp, Up, M, d, r, L, eps, terms, status_dev, st,
+                                   di.smem_optin, spin_limit());
         if (rc == DLRB200_ERR_CUDA) g_last_cuda_error = int(cudaGetLastError());
         return rc;
     }

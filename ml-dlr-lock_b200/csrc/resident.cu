@@ -28,7 +28,16 @@
 //       against 184 for BC at d = 2048, 4 rows
 // Both are byte-counted st.async on the receiver's mbarrier: no fences.  Sums are fp32 in a fixed order: repeatable.
 //
-// Measured on a B200 against the best kernel before it (us): d = 1024 (clusters of 4), 1 / 8 / 264 rows: 110 / 111 / 124
+// Operands.  h and s are rounded to bf16 where they meet the weights, as in the striped kernels.  TERMS is the form for calls
+// that run in fp32 throughout otherwise (decode_cluster.cu): a value goes into the tensor core as three bf16 terms of 8 bits
+// each, which add up to it exactly.  A cluster has two rows there and a token tile eight columns, so the terms (column 4 row +
+// term) cost no further mma.sync: what they cost is adding up the columns (one shuffle for two words) and taking h and s
+// apart.  Two terms of a row are the two columns a lane holds of an accumulator, the third is in the lane beside it.  Error
+// against 64 bits, output rounding included: d = 1024, 64 rows 1.6574e-3, 6e-5 to 9e-5 of the values on the other side of a
+// tie, both as decode_cluster.cu (rounded operands: 1.7133e-3, 0.18); d = 2048, 28 rows 1.6673e-3 (1.7225e-3).  Time (us,
+// rounded operands / terms / decode_cluster.cu): d = 1024, 8 rows 109 / 117 / 294; d = 2048, 17 rows 150 / 162 / 394.
+//
+// Measured on a B200 against the best kernel before it (us): d = 1024 (clusters of 4), 1 / 8 / 264 rows: 110 / 117 / 124
 // against 281 / 295 / 751; d = 2048 (8), 4 / 64 / 333 rows: 150 / 162 / 380 against 333 / 767 / 886; d = 4096 (16), 1 / 16 /
 // 64 rows: 222 / 236 / 357 against 323 / 521 / 1092; d = 5120 (16), 12 / 64 / 112 rows: 648 / 735 / 870 against 828 / 2350 /
 // 5555.
@@ -58,7 +67,8 @@ struct RParams {
 };
 
 // NU warps own the columns of the stripe (U contraction, activations, exchange), NVW warps the rows of V'.
-template <int R, int W, int NU, int NT, bool BC, int CS>
+// TERMS: the form with operands of 24 bits (see the top of the file).
+template <int R, int W, int NU, int NT, bool BC, int CS, bool TERMS>
 struct RCfg {
     static constexpr int MT_V = R / 16, MT_U = W / 16;
     static constexpr int NVW = MT_V <= 4 ? MT_V : (R == 128 ? 4 : 8);
@@ -82,16 +92,20 @@ struct RCfg {
     static constexpr int HB_BYTES = KS_V * NT * 32 * 8;  // bf16 activations as B fragments [ks / 2][nt][lane][ks & 1]
     static constexpr int SB_BYTES = MP * SS * 2;
     // partial sums of squares, [row][warp * 8 + g]; the row stride keeps a warp's stores (4 row pairs x 8) apart
-    static constexpr int QN = (NU * 8 + 31) / 32 * 32;
+    // (TERMS: two rows, [row][warp * 16 + 2 g + half])
+    static constexpr int QN = TERMS ? NU * 16 : (NU * 8 + 31) / 32 * 32;
     static constexpr int QS = QN + 4;
-    static constexpr int SSP_BYTES = QS * MP * 4;
+    static constexpr int MAX_ROWS = TERMS ? 2 : MP;      // rows per cluster
+    static constexpr int SSP_BYTES = QS * MAX_ROWS * 4;
     // The partitions of z.  RS: owner slices of SW columns, [source][row pair][column][2] with a source stride that is
-    // 16 words off a multiple of 32 (two sources are read at once).  BC: [source][tile][token tile][lane][4].
+    // 16 words off a multiple of 32 (two sources are read at once).  BC: [source][tile][token tile][lane][4], TERMS
+    // [source][tile][lane].
     static constexpr int SW = R / CS;                    // columns of z per owner (RS)
-    static constexpr int SRC_F = BC ? MT_V * NT * 128 : NPAIR * SW * 2 + 16;   // floats of one source's block
+    static constexpr int SRC_F = BC ? MT_V * NT * (TERMS ? 32 : 128) : NPAIR * SW * 2 + 16;   // floats of one source's block
     static constexpr int RECV_F = (BC ? 2 : 1) * CS * SRC_F;
     static constexpr int FIXED_BYTES = HB_BYTES + SB_BYTES + SSP_BYTES + RECV_F * 4 + 2 * CS * MP * 4 + 1024 /*barriers*/ + 1024 /*alignment*/;
     static_assert(VM <= 2, "tiles of V' per warp");
+    static_assert(!TERMS || (NT == 1 && VM == 1 && UM == 2 && PREF && QN % 64 == 0), "a pair of lanes deals out 2 words of z and 4 of dh");
     static_assert(VBOXES % VB == 0 && MT_V % NVW == 0 && MT_U % NU == 0, "whole tiles");
 };
 
@@ -107,6 +121,18 @@ struct RBars {
 };
 static_assert(sizeof(RBars) <= 1024, "barrier block");
 
+// Sums over two neighbouring lanes, dealt out: the even one gets that of a, the odd one that of b.
+__device__ __forceinline__ float pair_deal(float a, float b, bool odd) {
+    return (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+}
+
+// What is left of v after its k leading terms of 8 bits each (k < 3): rounded to bf16, term k of v.
+__device__ __forceinline__ float after_terms(float v, int k) {
+    const float r1 = v - __bfloat162float(__float2bfloat16_rn(v));
+    const float r2 = r1 - __bfloat162float(__float2bfloat16_rn(r1));
+    return k == 0 ? v : (k == 1 ? r1 : r2);
+}
+
 // 8 x 8 transposition of packed 16-bit values across a warp
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     uint32_t r;
@@ -116,10 +142,10 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 
 __device__ __forceinline__ void bar_id(int id, int n) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
-template <int R, int W, int NU, int NT, bool BC, int CS>
-__global__ void __launch_bounds__(RCfg<R, W, NU, NT, BC, CS>::THREADS, 1)
+template <int R, int W, int NU, int NT, bool BC, int CS, bool TERMS>
+__global__ void __launch_bounds__(RCfg<R, W, NU, NT, BC, CS, TERMS>::THREADS, 1)
 dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmU, RParams p, int SV, int SU) {
-    using C = RCfg<R, W, NU, NT, BC, CS>;
+    using C = RCfg<R, W, NU, NT, BC, CS, TERMS>;
     constexpr int SW = C::SW, SRC_F = C::SRC_F, MP = C::MP;
     constexpr int UTHREADS = 32 * NU, ATHREADS = 32 * C::CWARPS;
     extern __shared__ uint8_t smem_raw[];
@@ -169,6 +195,8 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
     // operand rows past the batch never receive s; sums of squares of warps there are not
     for (int i = tid; i < C::SSP_BYTES / 4; i += C::THREADS) ssp[i] = 0.f;
     for (int i = tid; i < C::SB_BYTES / 4; i += C::THREADS) reinterpret_cast<uint32_t*>(sb)[i] = 0u;
+    if constexpr (TERMS)                                     // (columns 6 and 7 of the token tile)
+        for (int i = tid; i < C::HB_BYTES / 4; i += C::THREADS) reinterpret_cast<uint32_t*>(hb)[i] = 0u;
     __syncthreads();
     // the peers' barriers must exist before anyone sends to them
     cluster_arrive_release();
@@ -231,6 +259,9 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
         uint32_t voff[4];                                // k step k % 4 of a tile
 #pragma unroll
         for (int k = 0; k < 4; ++k) voff[k] = (16u * uint32_t(vw) + a_row) * 128u + ((uint32_t(k) * 32u + a_col) ^ ((a_row & 7u) << 4));
+        // (TERMS: the fragments of the second row's columns lie two by two the other way round, so that the stores of a
+        // column of both rows go to different banks)
+        const int hb_lane = TERMS ? lane ^ ((lane >> 4) << 2) : lane;
         uint32_t va[C::PREF ? C::KS_V : 1][4];
         auto stage_done = [&]() {
             __syncwarp();
@@ -259,11 +290,16 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
         // where this warp's partial z goes: BC the same block in every CTA, RS the owners of its two halves
         uint32_t peer_recv[BC ? CS : 2 * C::VM], peer_bar[BC ? CS : 2 * C::VM];
         if constexpr (BC) {
+            const int word = TERMS ? vw * 32 + lane : (vw * NT * 32 + lane) * 4;
 #pragma unroll
             for (int k = 0; k < CS; ++k) {
-                peer_recv[k] = mapa(recv_s + uint32_t(int(rank) * SRC_F + (vw * NT * 32 + lane) * 4) * 4u, uint32_t(k));
+                peer_recv[k] = mapa(recv_s + uint32_t(int(rank) * SRC_F + word) * 4u, uint32_t(k));
                 peer_bar[k] = mapa(smem_u32(&bars->rbar[0]), uint32_t(k));
             }
+        } else if constexpr (TERMS) {
+            const int col = 16 * vw + 8 * (t & 1) + g;
+            peer_recv[0] = mapa(recv_s + uint32_t(int(rank) * SRC_F + (col % SW) * 2 + (t >> 1)) * 4u, uint32_t(col / SW));
+            peer_bar[0] = mapa(smem_u32(&bars->rbar[0]), uint32_t(col / SW));
         } else {
 #pragma unroll
             for (int i = 0; i < 2 * C::VM; ++i) {
@@ -313,7 +349,7 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
                     if (k2 + 1 < C::KS_V / 2) fetch(k2 + 1);
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt) {
-                        const uint4 b = *reinterpret_cast<const uint4*>(hb + ((k2 * NT + nt) * 32 + lane) * 16);
+                        const uint4 b = *reinterpret_cast<const uint4*>(hb + ((k2 * NT + nt) * 32 + hb_lane) * 16);
                         mma_bf16_16816(zc[0][nt][(2 * k2) % C::CH], a0[0], a0[1], a0[2], a0[3], b.x, b.y);
                         mma_bf16_16816(zc[0][nt][(2 * k2 + 1) % C::CH], a1[0], a1[1], a1[2], a1[3], b.z, b.w);
                         if constexpr (C::VM > 1) {
@@ -367,7 +403,13 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
 #pragma unroll
                         for (int k = 1; k < C::CH; ++k) z[c] += zc[vm][nt][k][c];
                     }
-                    if (8 * nt + 2 * t < rows) {
+                    if constexpr (TERMS) {
+                        // add up the terms: two in this lane, two in the one beside it; row t / 2, column 8 (t % 2) + g is left
+                        const uint32_t word = __float_as_uint(pair_deal(z[0] + z[1], z[2] + z[3], t & 1));
+#pragma unroll
+                        for (int k = 0; k < (BC ? CS : 1); ++k)
+                            st_async_b32(peer_recv[k] + (BC ? par * uint32_t(CS * SRC_F * 4) : 0u), word, peer_bar[k] + (BC ? 8u * par : 0u));
+                    } else if (8 * nt + 2 * t < rows) {
                         if constexpr (BC) {
 #pragma unroll
                             for (int k = 0; k < CS; ++k)
@@ -398,43 +440,66 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
         }
     } else {
         // =============================== U warps ====================================
-        float h[C::UM][NT][4];       // columns stripe0 + 16 u + g (+8), rows 8 nt + 2t, + 1 of this cluster's rows
+        // columns stripe0 + 16 u + g (+8), rows 8 nt + 2t, + 1 of this cluster's rows; TERMS: h[i][0][0] only, columns
+        // stripe0 + 16 u + 8 (t % 2) + g of row t / 2
+        float h[C::UM][NT][4];
+        const int row_t = t >> 1, col_t = stripe0 + 32 * warp + 8 * (t & 1) + g;
+        if constexpr (TERMS) {
 #pragma unroll
-        for (int i = 0; i < C::UM; ++i)
+            for (int i = 0; i < 2; ++i) h[i][0][0] = row_t < rows ? __bfloat162float(p.x[size_t(row0 + row_t) * p.d + col_t + 16 * i]) : 0.f;
+        } else {
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
+            for (int i = 0; i < C::UM; ++i)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int row = 8 * nt + 2 * t + (c & 1);
-                    const int col = stripe0 + 16 * (warp * C::UM + i) + g + 8 * (c >> 1);
-                    h[i][nt][c] = row < rows ? __bfloat162float(p.x[size_t(row0 + row) * p.d + col]) : 0.f;
-                }
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const int row = 8 * nt + 2 * t + (c & 1);
+                        const int col = stripe0 + 16 * (warp * C::UM + i) + g + 8 * (c >> 1);
+                        h[i][nt][c] = row < rows ? __bfloat162float(p.x[size_t(row0 + row) * p.d + col]) : 0.f;
+                    }
+        }
         // activations (bf16, as B fragments) and sums of squares for the next layer
         auto publish = [&]() {
+            if constexpr (TERMS) {
+                float v[2] = {h[0][0][0], h[1][0][0]};
+                ssp[row_t * C::QS + warp * 16 + 2 * g + (t & 1)] = v[0] * v[0] + v[1] * v[1];
+                // B fragments: K row 16 i + 8 (t % 2) + g of this warp's 32, column 4 row + term of the token tile (see hb_lane)
+                uint8_t* at = hb + warp * 512 + (g >> 1) * 16 + 4 * (t & 1) + 2 * (g & 1);
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                float q0 = 0.f, q1 = 0.f;
+                for (int k = 0; k < 3; ++k)
 #pragma unroll
-                for (int i = 0; i < C::UM; ++i) {
-                    const float* a = h[i][nt];
-                    q0 += a[0] * a[0] + a[2] * a[2];
-                    q1 += a[1] * a[1] + a[3] * a[3];
-                }
-                ssp[(8 * nt + 2 * t) * C::QS + warp * 8 + g] = q0;
-                ssp[(8 * nt + 2 * t + 1) * C::QS + warp * 8 + g] = q1;
+                    for (int i = 0; i < 2; ++i) {
+                        const __nv_bfloat16 b = __float2bfloat16_rn(v[i]);
+                        *reinterpret_cast<__nv_bfloat16*>(at + 64 * (row_t ? 4 + (k ^ 1) : k) + 8 * i) = b;
+                        v[i] -= __bfloat162float(b);
+                    }
+            } else {
 #pragma unroll
-                for (int i = 0; i < C::UM; i += 2) {
-                    const int ks = warp * C::UM + i;
-                    uint4 b;
-                    b.x = movmatrix_trans(pack_bf16x2(h[i][nt][0], h[i][nt][1]));
-                    b.y = movmatrix_trans(pack_bf16x2(h[i][nt][2], h[i][nt][3]));
-                    if constexpr (C::UM % 2 == 0) {
-                        b.z = movmatrix_trans(pack_bf16x2(h[(i + 1) % C::UM][nt][0], h[(i + 1) % C::UM][nt][1]));
-                        b.w = movmatrix_trans(pack_bf16x2(h[(i + 1) % C::UM][nt][2], h[(i + 1) % C::UM][nt][3]));
-                        *reinterpret_cast<uint4*>(hb + ((ks / 2 * NT + nt) * 32 + lane) * 16) = b;
-                    } else {
-                        static_assert(C::UM == 1 || C::UM % 2 == 0, "column tiles per warp");
-                        *reinterpret_cast<uint2*>(hb + ((ks / 2 * NT + nt) * 32 + lane) * 16 + (ks & 1) * 8) = make_uint2(b.x, b.y);
+                for (int nt = 0; nt < NT; ++nt) {
+                    float q0 = 0.f, q1 = 0.f;
+#pragma unroll
+                    for (int i = 0; i < C::UM; ++i) {
+                        const float* a = h[i][nt];
+                        q0 += a[0] * a[0] + a[2] * a[2];
+                        q1 += a[1] * a[1] + a[3] * a[3];
+                    }
+                    ssp[(8 * nt + 2 * t) * C::QS + warp * 8 + g] = q0;
+                    ssp[(8 * nt + 2 * t + 1) * C::QS + warp * 8 + g] = q1;
+#pragma unroll
+                    for (int i = 0; i < C::UM; i += 2) {
+                        const int ks = warp * C::UM + i;
+                        uint4 b;
+                        b.x = movmatrix_trans(pack_bf16x2(h[i][nt][0], h[i][nt][1]));
+                        b.y = movmatrix_trans(pack_bf16x2(h[i][nt][2], h[i][nt][3]));
+                        if constexpr (C::UM % 2 == 0) {
+                            b.z = movmatrix_trans(pack_bf16x2(h[(i + 1) % C::UM][nt][0], h[(i + 1) % C::UM][nt][1]));
+                            b.w = movmatrix_trans(pack_bf16x2(h[(i + 1) % C::UM][nt][2], h[(i + 1) % C::UM][nt][3]));
+                            *reinterpret_cast<uint4*>(hb + ((ks / 2 * NT + nt) * 32 + lane) * 16) = b;
+                        } else {
+                            static_assert(C::UM == 1 || C::UM % 2 == 0, "column tiles per warp");
+                            *reinterpret_cast<uint2*>(hb + ((ks / 2 * NT + nt) * 32 + lane) * 16 + (ks & 1) * 8) = make_uint2(b.x, b.y);
+                        }
                     }
                 }
             }
@@ -452,7 +517,7 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             rp.step(uint32_t(SU));
         };
         const uint32_t sbar_s = smem_u32(&bars->sbar);
-        const uint32_t z_bytes = BC ? uint32_t(CS * C::MT_V * 8 * 16) * uint32_t(pairs) : uint32_t(CS * SW * 8) * uint32_t(pairs);
+        const uint32_t z_bytes = BC ? (TERMS ? uint32_t(CS * R * 8) : uint32_t(CS * C::MT_V * 8 * 16) * uint32_t(pairs)) : uint32_t(CS * SW * 8) * uint32_t(pairs);
         const uint32_t q_dst = mapa(recvq_s + uint32_t(int(rank) * MP) * 4u, uint32_t(lane % CS));      // lane -> peer
         const uint32_t q_bar = mapa(smem_u32(&bars->rbar[0]), uint32_t(lane % CS));
         const uint32_t sb_b = sb_s + uint32_t((lane & 7) * C::SS + (lane >> 3) * 8) * 2u;      // ldmatrix of s
@@ -473,23 +538,23 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             const bool stop = layer_barrier(l);
             // ---- sums of squares: a row per warp, lane -> every eighth 16 bytes of its NU * 8 partial sums, then -> peer
 #pragma unroll
-            for (int row = warp; row < MP; row += NU) {
+            for (int row = warp; row < C::MAX_ROWS; row += NU) {
                 if (row < rows) {
+                    constexpr int QL = TERMS ? 16 : 8;           // lanes with different words
                     float q = 0.f;
 #pragma unroll
-                    for (int i = 0; i < C::QN / 32; ++i) {
-                        const float4 f = *reinterpret_cast<const float4*>(ssp + row * C::QS + 32 * i + 4 * (lane & 7));
+                    for (int i = 0; i < C::QN / (4 * QL); ++i) {
+                        const float4 f = *reinterpret_cast<const float4*>(ssp + row * C::QS + 4 * QL * i + 4 * (lane % QL));
                         q += (f.x + f.y) + (f.z + f.w);
                     }
-                    q += __shfl_xor_sync(0xffffffffu, q, 1);
-                    q += __shfl_xor_sync(0xffffffffu, q, 2);
-                    q += __shfl_xor_sync(0xffffffffu, q, 4);
+#pragma unroll
+                    for (int o = 1; o < QL; o <<= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
                     if (lane < CS) st_async_b32(q_dst + uint32_t((int(par) * CS * MP + row) * 4), __float_as_uint(q), q_bar + 8u * par);
                 }
             }
             if (warp == NU - 1 && lane == 0) {
                 mbar_arrive_expect_tx(rbar_s, z_bytes + uint32_t(CS * 4 * rows));
-                if (!BC) mbar_arrive_expect_tx(sbar_s, uint32_t(rows * R * 2));
+                if (!BC) mbar_arrive_expect_tx(sbar_s, uint32_t(rows * R * 2) * (TERMS ? 3u : 1u));
                 if (*reinterpret_cast<volatile int*>(&bars->give_up)) err = DLRB200_ERR_TIMEOUT_BARRIER;
             }
             // ---- this layer's U' fragments, while the V warps work and the partials travel
@@ -516,21 +581,27 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             if constexpr (BC) {
                 // ---- every CTA: add up all partials of z; thread -> the same word of every source's block
                 static_assert(NT == 1 || !BC, "one token tile");
-                constexpr int ITS = (C::MT_V * 128 + UTHREADS - 1) / UTHREADS;
-                const int c = tid & 3, ln = (tid >> 2) & 31;
-                const int row = 2 * (ln & 3) + (c & 1);
+                // (TERMS: one word of z per lane of a tile, every term of s stored by other warps)
+                constexpr int WORDS = SRC_F, ITS = TERMS ? 1 : (WORDS + UTHREADS - 1) / UTHREADS;
+                static_assert(!TERMS || (WORDS % 32 == 0 && 3 * WORDS <= UTHREADS), "a thread per word and term");
+                const int c = tid & 3, ln = TERMS ? lane : (tid >> 2) & 31;
+                const int row = TERMS ? row_t : 2 * (ln & 3) + (c & 1), term = TERMS ? tid / WORDS : 0;
                 float q = 0.f;
 #pragma unroll
                 for (int k = 0; k < CS; ++k) q += recvq[(int(par) * CS + k) * MP + row];
                 const float rstd = rsqrtf(q * p.inv_d + p.eps);
 #pragma unroll
                 for (int it = 0; it < ITS; ++it) {
-                    const int e = tid + it * UTHREADS;
-                    if (row < rows && e < C::MT_V * 128) {
+                    const int e = TERMS ? tid % WORDS : tid + it * UTHREADS;
+                    if (row < rows && (TERMS ? term < 3 : e < WORDS)) {
                         float z = 0.f;
 #pragma unroll
                         for (int k = 0; k < CS; ++k) z += recv[(int(par) * CS + k) * SRC_F + e];
-                        reinterpret_cast<__nv_bfloat16*>(sb)[row * C::SS + 16 * (e >> 7) + (ln >> 2) + 8 * (c >> 1)] = __float2bfloat16_rn(silu_f(z * rstd));
+                        const float s = silu_f(z * rstd);
+                        if constexpr (TERMS)
+                            reinterpret_cast<__nv_bfloat16*>(sb)[(4 * row + term) * C::SS + 16 * (e >> 5) + 8 * (t & 1) + g] = __float2bfloat16_rn(after_terms(s, term));
+                        else
+                            reinterpret_cast<__nv_bfloat16*>(sb)[row * C::SS + 16 * (e >> 7) + (ln >> 2) + 8 * (c >> 1)] = __float2bfloat16_rn(s);
                     }
                 }
                 bar_id(2, UTHREADS);                         // s is complete
@@ -567,6 +638,24 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
                             z1 += __shfl_xor_sync(0xffffffffu, z1, o);
                         }
                         // two columns of one row per lane: even lanes the first row of the pair, odd lanes the second
+                        if constexpr (TERMS) {
+                            const float s0 = silu_f(z0 * rstd[it][0]), s1 = silu_f(z1 * rstd[it][1]);
+                            const float other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? s0 : s1, 1);
+                            float a = (lane & 1) ? other : s0, b = (lane & 1) ? s1 : other;
+                            if ((lane & 1) < rows) {
+                                const uint32_t dst = sb_s + uint32_t((lane & 1) * 4 * C::SS + int(rank) * SW + (zl & ~1)) * 2u;
+#pragma unroll
+                                for (int term = 0; term < 3; ++term) {
+                                    const uint32_t v = pack_bf16x2(a, b);
+                                    a -= bf16lo_to_f(v);
+                                    b -= bf16hi_to_f(v);
+#pragma unroll
+                                    for (int k = 0; k < PER; ++k)
+                                        st_async_b32(dst + uint32_t(term * C::SS) * 2u + to_peer[k], v, sbar_s + to_peer[k]);
+                                }
+                            }
+                            continue;
+                        }
                         const uint32_t mine = pack_bf16x2(silu_f(z0 * rstd[it][0]), silu_f(z1 * rstd[it][1]));
                         const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1);
                         const uint32_t v = (lane & 1) ? __byte_perm(other, mine, 0x7632) : __byte_perm(mine, other, 0x5410);
@@ -636,26 +725,44 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
                     stage_done();
                 }
             }
+            if constexpr (TERMS) {
+                // add up the terms of dh as those of z
 #pragma unroll
-            for (int i = 0; i < C::UM; ++i)
+                for (int i = 0; i < 2; ++i) {
+                    float dh[2];
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
+                    for (int hh = 0; hh < 2; ++hh)
+                        dh[hh] = (uc[i][0][0][2 * hh] + uc[i][0][0][2 * hh + 1]) + (uc[i][0][UCH - 1][2 * hh] + uc[i][0][UCH - 1][2 * hh + 1]);
+                    h[i][0][0] += pair_deal(dh[0], dh[1], t & 1);
+                }
+            } else {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) h[i][nt][c] += UCH == 2 ? uc[i][nt][0][c] + uc[i][nt][UCH - 1][c] : uc[i][nt][0][c];
+                for (int i = 0; i < C::UM; ++i)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) h[i][nt][c] += UCH == 2 ? uc[i][nt][0][c] + uc[i][nt][UCH - 1][c] : uc[i][nt][0][c];
+            }
             if (stop) break;
             if (l + 1 < p.L) publish();
         }
         if (l >= p.L && !err) {
+            if constexpr (TERMS) {
 #pragma unroll
-            for (int i = 0; i < C::UM; ++i)
+                for (int i = 0; i < 2; ++i)
+                    if (row_t < rows) p.y[size_t(row0 + row_t) * p.d + col_t + 16 * i] = __float2bfloat16_rn(h[i][0][0]);
+            } else {
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
+                for (int i = 0; i < C::UM; ++i)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const int row = 8 * nt + 2 * t + (c & 1);
-                        const int col = stripe0 + 16 * (warp * C::UM + i) + g + 8 * (c >> 1);
-                        if (row < rows) p.y[size_t(row0 + row) * p.d + col] = __float2bfloat16_rn(h[i][nt][c]);
-                    }
+                    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const int row = 8 * nt + 2 * t + (c & 1);
+                            const int col = stripe0 + 16 * (warp * C::UM + i) + g + 8 * (c >> 1);
+                            if (row < rows) p.y[size_t(row0 + row) * p.d + col] = __float2bfloat16_rn(h[i][nt][c]);
+                        }
+            }
         }
     }
     if (err) {
@@ -681,6 +788,7 @@ struct RArgs {
     cudaStream_t stream;
     int smem_optin;
     unsigned int spin_limit;
+    bool terms;                 // operands of 24 bits
 };
 
 // How a call would be cut up: token tiles per cluster, rows per cluster, clusters at once, estimated time.
@@ -692,9 +800,9 @@ struct RShape {
 
 constexpr int kMaxDevices = 64;
 
-template <int R, int W, int NU, int NT, bool BC, int CS>
+template <int R, int W, int NU, int NT, bool BC, int CS, bool TERMS = false>
 struct RLaunch {
-    using C = RCfg<R, W, NU, NT, BC, CS>;
+    using C = RCfg<R, W, NU, NT, BC, CS, TERMS>;
     int SV = 0, SU = 0, smem = 0;
 
     // Both rings as deep as fits, alike in layers.  The fragments of a layer are taken before the layer: with prefetching a
@@ -732,7 +840,7 @@ struct RLaunch {
         if (!smem || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
         int n = known[dev].load(std::memory_order_acquire);
         if (n != 0) return n;
-        auto kern = dlr_resident_kernel<R, W, NU, NT, BC, CS>;
+        auto kern = dlr_resident_kernel<R, W, NU, NT, BC, CS, TERMS>;
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         config(cfg, attr, 1, nullptr);
@@ -753,7 +861,7 @@ struct RLaunch {
         if (mc < 1) return;
         int rows = (M + mc - 1) / mc;
         rows = rows < 2 ? 2 : (rows + 1) & ~1;
-        if (rows > C::MP) rows = C::MP;
+        if (rows > C::MAX_ROWS) rows = C::MAX_ROWS;
         const int clusters = (M + rows - 1) / rows, waves = (clusters + mc - 1) / mc;
         const double us = double(waves) * L * us_per_layer;
         if (us < best.us) {
@@ -780,15 +888,25 @@ struct RLaunch {
         if (!encode_2d_bf16(a.enc, &tmV, a.Vp, uint64_t(a.d), uint64_t(a.L) * R, 64, R, 128) ||
             !encode_2d_bf16(a.enc, &tmU, a.Up, uint64_t(R), uint64_t(a.L) * a.d, C::KW, W > 256 ? W / 2 : W, C::KW * 2))
             return DLRB200_ERR_CUDA;
-        const cudaError_t ce = cudaLaunchKernelEx(&cfg, dlr_resident_kernel<R, W, NU, NT, BC, CS>, tmV, tmU, p, SV, SU);
+        const cudaError_t ce = cudaLaunchKernelEx(&cfg, dlr_resident_kernel<R, W, NU, NT, BC, CS, TERMS>, tmV, tmU, p, SV, SU);
         return ce == cudaSuccess ? DLRB200_OK : DLRB200_ERR_CUDA;
     }
 };
 
 // One shape of net: three kernels (8, 16 or 32 rows per cluster) with their time per layer, microseconds, measured on a
-// B200 with every resident cluster at work.
+// B200 with every resident cluster at work; and the one with operands of 24 bits (two rows per cluster, time tt) where there is
+// one.
 template <int R, int W, int NU, int CS, bool BC>
-int shape_call(const RArgs& a, double t1, double t2, double t4, RShape& best, bool launch) {
+int shape_call(const RArgs& a, double t1, double t2, double t4, double tt, RShape& best, bool launch) {
+    if (a.terms) {
+        if constexpr (R <= 64) {
+            const RLaunch<R, W, NU, 1, BC, CS, true> k(a.smem_optin);
+            k.consider(a.M, a.L, tt, best);
+            if (best.nt == 0) return DLRB200_ERR_UNSUPPORTED_SHAPE;
+            return launch ? k.launch(a, best) : DLRB200_OK;
+        }
+        return DLRB200_ERR_UNSUPPORTED_SHAPE;
+    }
     const RLaunch<R, W, NU, 1, BC, CS> k1(a.smem_optin);
     const RLaunch<R, W, NU, 2, false, CS> k2(a.smem_optin);
     const RLaunch<R, W, NU, 4, false, CS> k4(a.smem_optin);
@@ -801,10 +919,10 @@ int shape_call(const RArgs& a, double t1, double t2, double t4, RShape& best, bo
 }
 
 int dispatch_resident(const RArgs& a, int r, RShape& best, bool launch) {
-    if (r == 32 && a.d == 1024) return shape_call<32, 256, 8, 4, true>(a, 0.84, 1.26, 2.19, best, launch);
-    if (r == 64 && a.d == 2048) return shape_call<64, 256, 8, 8, false>(a, 1.20, 1.82, 2.95, best, launch);
-    if (r == 128 && a.d == 4096) return shape_call<128, 256, 8, 16, false>(a, 1.80, 2.78, 4.74, best, launch);
-    if (r == 256 && a.d == 5120) return shape_call<256, 320, 10, 16, false>(a, 4.60, 5.84, 10.9, best, launch);
+    if (r == 32 && a.d == 1024) return shape_call<32, 256, 8, 4, true>(a, 0.84, 1.26, 2.19, 0.83, best, launch);
+    if (r == 64 && a.d == 2048) return shape_call<64, 256, 8, 8, false>(a, 1.20, 1.82, 2.95, 1.16, best, launch);
+    if (r == 128 && a.d == 4096) return shape_call<128, 256, 8, 16, false>(a, 1.80, 2.78, 4.74, 0.0, best, launch);
+    if (r == 256 && a.d == 5120) return shape_call<256, 320, 10, 16, false>(a, 4.60, 5.84, 10.9, 0.0, best, launch);
     return DLRB200_ERR_UNSUPPORTED_SHAPE;
 }
 
@@ -814,9 +932,9 @@ bool resident_supported(int d, int r) {
     return (r == 32 && d == 1024) || (r == 64 && d == 2048) || (r == 128 && d == 4096) || (r == 256 && d == 5120);
 }
 
-double resident_estimate_us(int M, int d, int r, int L, int smem_optin, dlrb200_plan* plan) {
+double resident_estimate_us(int M, int d, int r, int L, bool terms, int smem_optin, dlrb200_plan* plan) {
     RArgs a{};
-    a.M = M; a.d = d; a.L = L; a.smem_optin = smem_optin;
+    a.M = M; a.d = d; a.L = L; a.smem_optin = smem_optin; a.terms = terms;
     RShape sh;
     if (dispatch_resident(a, r, sh, false) != DLRB200_OK) return 1e30;
     if (plan) {
@@ -833,8 +951,8 @@ double resident_estimate_us(int M, int d, int r, int L, int smem_optin, dlrb200_
 }
 
 int resident_forward(void* enc, const void* x, void* y, const void* Vp, const void* Up, int M, int d, int r, int L,
-                     float eps, int* status_dev, cudaStream_t stream, int smem_optin, unsigned int spin_limit) {
-    RArgs a{enc, x, y, Vp, Up, M, d, L, eps, status_dev, stream, smem_optin, spin_limit};
+                     float eps, bool terms, int* status_dev, cudaStream_t stream, int smem_optin, unsigned int spin_limit) {
+    RArgs a{enc, x, y, Vp, Up, M, d, L, eps, status_dev, stream, smem_optin, spin_limit, terms};
     RShape sh;
     return dispatch_resident(a, r, sh, true);
 }

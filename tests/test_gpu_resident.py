@@ -9,7 +9,7 @@ from oracle import dlrnet_oracle as O
 
 pytestmark = pytest.mark.gpu
 
-# Activations in fp32, operands rounded to bf16, as in the other small-batch kernels: same gates.
+# Activations in fp32, operands rounded to bf16, as in the striped kernels: same gates.
 TOL_TOTAL, TOL_UPDATE = 5e-3, 2e-2
 
 CASES = [(1024, 32, 5, M) for M in (1, 2, 3, 8, 9, 63, 267, 530, 1100)]
@@ -38,6 +38,30 @@ def test_resident_kernel(d, r, L, M, monkeypatch):
     want = O.forward_fp32(x, p)
     assert O.rel_l2(y1.cpu(), want) <= TOL_TOTAL
     assert O.rel_l2_update_q(y1.cpu(), want, x) <= TOL_UPDATE
+
+
+# Calls whose any-shape kernel works in fp32 throughout (one cluster per pair of rows): operands of three bf16 terms here.
+# One row and two in the last cluster, one cluster and several, one layer.  The result is that of 64 bits rounded once, but
+# for ties: an error e before the rounding moves at most 512 e of the values to their neighbour (a bf16 spacing is at least
+# 2^-8 of a value), and e is about 1e-6 for fp32 sums of 256 products over the layers here.  Operands of 8 bits move 5 to 18 %.
+@pytest.mark.parametrize("d,r,L,M", [(1024, 32, 1, 2), (1024, 32, 141, 2), (1024, 32, 4, 3), (1024, 32, 20, 8), (1024, 32, 7, 63), (1024, 32, 30, 64),
+                                     (2048, 64, 1, 17), (2048, 64, 142, 17), (2048, 64, 20, 28), (2048, 64, 5, 27)])
+def test_pair_of_rows_in_fp32(d, r, L, M):
+    import dlr_lock_b200 as D
+    dev = torch.device("cuda:0")
+    p, x = O.seeded_case(d, r, L, M, seed=d + L + M, alpha=1.0, gain_jitter=0.1)
+    Vf, Uf = D.ops.fold_weights(p.V.to(dev), p.U.to(dev), p.w.to(dev), p.alpha.to(dev))
+    y = D.ops.forward_folded(x.to(dev), Vf, Uf, p.eps)
+    again = D.ops.forward_folded(x.to(dev), Vf, Uf, p.eps)
+    torch.cuda.synchronize()
+    D.ops.check_status()
+    assert torch.equal(y, again)
+    h = x.to(dev).double()
+    for V, U in zip(Vf.double(), Uf.double()):
+        z = (h @ V.T) * torch.rsqrt(h.square().mean(-1, keepdim=True) + p.eps)
+        h = h + torch.nn.functional.silu(z) @ U.T
+    assert (y != h.to(torch.bfloat16)).double().mean() <= 1e-3
+    assert O.rel_l2(y.double(), h) <= 1.01 * O.rel_l2(h.to(torch.bfloat16), h)
 
 
 def test_resident_kernel_gives_up_while_the_status_word_is_set(monkeypatch):
