@@ -35,7 +35,7 @@
 // apart.  Two terms of a row are the two columns a lane holds of an accumulator, the third is in the lane beside it.  Error
 // against 64 bits, output rounding included: d = 1024, 64 rows 1.6574e-3, 6e-5 to 9e-5 of the values on the other side of a
 // tie, both as decode_cluster.cu (rounded operands: 1.7133e-3, 0.18); d = 2048, 28 rows 1.6673e-3 (1.7225e-3).  Time (us,
-// rounded operands / terms / decode_cluster.cu): d = 1024, 8 rows 109 / 117 / 294; d = 2048, 17 rows 150 / 162 / 394.
+// rounded operands / terms / decode_cluster.cu): d = 1024, 8 rows 110 / 117 / 294; d = 2048, 17 rows 150 / 166 / 394.
 //
 // Measured on a B200 against the best kernel before it (us): d = 1024 (clusters of 4), 1 / 8 / 264 rows: 110 / 117 / 124
 // against 281 / 295 / 751; d = 2048 (8), 4 / 64 / 333 rows: 150 / 162 / 380 against 333 / 767 / 886; d = 4096 (16), 1 / 16 /
@@ -204,9 +204,13 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
 
     int err = 0;               // why this warp gave up
     const uint32_t flag_s = smem_u32(&bars->abort_flag);
-    auto wait_for = [&](uint32_t bar, uint32_t parity, int code, bool remote) {
-        const bool ok = remote ? mbar_wait_flag_cluster(bar, parity, flag_s, p.spin_limit) : mbar_wait_flag(bar, parity, flag_s, p.spin_limit);
+    auto wait_for = [&](uint32_t bar, uint32_t parity, int code, bool remote) {          // whole warps
+        const bool ok = remote ? mbar_wait_warp_cluster(bar, parity, flag_s, p.spin_limit) : mbar_wait_warp(bar, parity, flag_s, p.spin_limit);
         err = ok ? err : code;
+    };
+    auto wait_free = [&](uint64_t& bar, uint32_t parity) {                               // the producer's lane
+        if (!mbar_wait_lane(smem_u32(&bar), parity, flag_s, p.spin_limit)) err = DLRB200_ERR_TIMEOUT_COPY;
+        return err == 0;
     };
 
     // ---- weight rings: one thread asks for the tiles, in the order they are used
@@ -214,8 +218,7 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
     int vl = 0, vi = 0, ul = 0, ui = 0;                 // layer and stage in it asked for next
     auto ask_v = [&]() {
         if (vl >= p.L) return;
-        wait_for(smem_u32(&bars->v_empty[vq.st]), vq.ph ^ 1u, DLRB200_ERR_TIMEOUT_COPY, false);
-        if (err) return;
+        if (!wait_free(bars->v_empty[vq.st], vq.ph ^ 1u)) return;
         const uint32_t bar = smem_u32(&bars->v_full[vq.st]), dst = vring_s + vq.st * C::V_STAGE;
         mbar_arrive_expect_tx(bar, C::V_STAGE);
 #pragma unroll
@@ -226,8 +229,7 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
     };
     auto ask_u = [&]() {
         if (ul >= p.L) return;
-        wait_for(smem_u32(&bars->u_empty[uq.st]), uq.ph ^ 1u, DLRB200_ERR_TIMEOUT_COPY, false);
-        if (err) return;
+        if (!wait_free(bars->u_empty[uq.st], uq.ph ^ 1u)) return;
         const uint32_t bar = smem_u32(&bars->u_full[uq.st]), dst = uring_s + uq.st * C::U_STAGE;
         mbar_arrive_expect_tx(bar, C::U_STAGE);
         constexpr int UBR = W > 256 ? W / 2 : W;        // a box has at most 256 rows
@@ -557,6 +559,7 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
                 if (!BC) mbar_arrive_expect_tx(sbar_s, uint32_t(rows * R * 2) * (TERMS ? 3u : 1u));
                 if (*reinterpret_cast<volatile int*>(&bars->give_up)) err = DLRB200_ERR_TIMEOUT_BARRIER;
             }
+            __syncwarp();
             // ---- this layer's U' fragments, while the V warps work and the partials travel
             if constexpr (C::PREF) {
                 // (wide layers: not before the V warps are done, whose loads would queue behind these in the one port)
