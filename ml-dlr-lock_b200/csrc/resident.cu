@@ -438,7 +438,8 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
                 // the status word was set before this launch: give up
                 if (l == 0 && *reinterpret_cast<volatile int*>(p.status) != 0) *reinterpret_cast<volatile int*>(&bars->give_up) = 1;
             }
-            if (err || *abort_flag) drain_copies();
+            // (whatever the others do: they may give up after this, with copies still on their way)
+            drain_copies();
         }
     } else {
         // =============================== U warps ====================================

@@ -64,13 +64,19 @@ def test_pair_of_rows_in_fp32(d, r, L, M):
     assert O.rel_l2(y.double(), h) <= 1.01 * O.rel_l2(h.to(torch.bfloat16), h)
 
 
-def test_resident_kernel_gives_up_while_the_status_word_is_set(monkeypatch):
+# every kernel of every shape, on stacks that may be asked for whole before anyone gives up: copies still land while the rest
+# leaves
+@pytest.mark.parametrize("L", [6])
+@pytest.mark.parametrize("d,r,M", [(1024, 32, 1), (1024, 32, 8), (1024, 32, 267), (1024, 32, 530), (1024, 32, 1100), (2048, 64, 4), (2048, 64, 20),
+                                   (2048, 64, 200), (2048, 64, 400), (4096, 128, 1), (4096, 128, 115), (4096, 128, 200), (5120, 256, 3),
+                                   (5120, 256, 115), (5120, 256, 200)])
+def test_resident_kernel_gives_up_while_the_status_word_is_set(d, r, L, M, monkeypatch):
     # the word an earlier kernel would have left behind, set by the host: the call returns, leaves its output and the word
     # alone, and the next call on a cleared word works
     import dlr_lock_b200 as D
     monkeypatch.setenv("DLRB200_FORCE_PATH", "7")
     dev = torch.device("cuda:0")
-    p, x = O.seeded_case(2048, 64, 4, 20, seed=9, alpha=1.0, gain_jitter=0.1)
+    p, x = O.seeded_case(d, r, L, M, seed=9, alpha=1.0, gain_jitter=0.1)
     Vf, Uf = D.ops.fold_weights(p.V.to(dev), p.U.to(dev), p.w.to(dev), p.alpha.to(dev))
     xd = x.to(dev)
     D.ops.forward_folded(xd, Vf, Uf)
@@ -83,7 +89,7 @@ def test_resident_kernel_gives_up_while_the_status_word_is_set(monkeypatch):
     lib = D.ops._lib.load()
     vp = lambda t: ctypes.c_void_p(t.data_ptr())                    # (the tensor call would raise before it launches)
     st = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-    assert lib.dlrb200_forward(vp(xd), vp(out), vp(Vf), vp(Uf), 20, 2048, 64, 4, 1e-6, vp(ent.ws), ent.ws.numel(), vp(ent.status), st) == 0
+    assert lib.dlrb200_forward(vp(xd), vp(out), vp(Vf), vp(Uf), M, d, r, L, 1e-6, vp(ent.ws), ent.ws.numel(), vp(ent.status), st) == 0
     torch.cuda.synchronize()
     assert bool((out == 7.0).all())
     with pytest.raises(D.ops._lib.DlrB200Error):
@@ -92,3 +98,4 @@ def test_resident_kernel_gives_up_while_the_status_word_is_set(monkeypatch):
     torch.cuda.synchronize()
     D.ops.check_status()
     assert O.rel_l2(y.cpu(), O.forward_fp32(x, p)) <= TOL_TOTAL
+
