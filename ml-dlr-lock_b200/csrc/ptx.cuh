@@ -129,32 +129,33 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 // assembly with uniform branches: a look at a phase that is already complete costs about 60 cycles against 100 for the same
 // loop in C++ (measured; the difference is the bookkeeping for lanes that leave a loop at different times).  The branches are
 // uniform because the lanes vote on what they saw: a try_wait may give lanes different answers, and what follows in the
-// callers (mma.sync, ldmatrix, shuffles) needs the whole warp.  In the resident kernel the votes cost 0 to 3 % (us, without /
-// with: d = 1024, 8 rows 117.2 / 117.4; d = 2048, 4 rows 146.0 / 149.6; d = 4096, 16 rows 230 / 233).  `limit` must not be 0.
-#define DLR_MBAR_WAIT(NAME, FORM, AGREE1, AGREE2)                                                                   \
+// callers (mma.sync, ldmatrix, shuffles) needs the whole warp.  The flag needs no vote of its own: the warp, converged by the
+// one before, reads the one word in one instruction.  Measured (us, no votes / this / a vote on the flag too): d = 1024, one
+// row 111 / 103 / 109; d = 2048, 4 rows 146 / 146 / 150; d = 4096, 16 rows 233 / 236 / 237.  `limit` must not be 0.
+#define DLR_MBAR_WAIT(NAME, FORM, AGREE)                                                                            \
     __device__ __forceinline__ bool NAME(uint32_t bar, uint32_t parity, uint32_t flag, uint32_t limit) {            \
         uint32_t ok;                                                                                                \
         asm volatile(                                                                                               \
             "{\n\t.reg .pred P1, P2;\n\t.reg .u32 n, f;\n\tmov.u32 n, %4;\n"                                          \
-            "DLR_WAIT_%=:\n\t" FORM " P1, [%1], %2;\n\t" AGREE1 "@P1 bra.uni DLR_DONE_%=;\n\t"                           \
+            "DLR_WAIT_%=:\n\t" FORM " P1, [%1], %2;\n\t" AGREE "@P1 bra.uni DLR_DONE_%=;\n\t"                           \
             "ld.volatile.shared.u32 f, [%3];\n\tsub.u32 n, n, 1;\n\tsetp.ne.u32 P2, n, 0;\n\t"                      \
-            "setp.eq.and.u32 P2, f, 0, P2;\n\t" AGREE2 "@P2 bra.uni DLR_WAIT_%=;\n"                                  \
+            "setp.eq.and.u32 P2, f, 0, P2;\n\t@P2 bra.uni DLR_WAIT_%=;\n"                                  \
             "DLR_DONE_%=:\n\tselp.u32 %0, 1, 0, P1;\n\t}"                                                           \
             : "=r"(ok)                                                                                              \
             : "r"(bar), "r"(parity), "r"(flag), "r"(limit)                                                          \
             : "memory");                                                                                            \
         return ok != 0;                                                                                             \
     }
-#define DLR_AGREE(P) "vote.sync.all.pred " P ", " P ", 0xffffffff;\n\t"
+#define DLR_AGREE "vote.sync.all.pred P1, P1, 0xffffffff;\n\t"
 // For a whole warp, which leaves with one answer.  The warps of the tensor-core kernels wait with these, the issuing warps
 // too, which elect a lane only for the instructions of a chunk: a look by one lane of a split warp costs about 250 cycles.
 // Measured in the cluster kernel (us, issue and copy warps as one elected thread / whole): d = 1024, 4096 rows 482 / 454;
 // d = 4096, 1000 rows 1136 / 1064.
-DLR_MBAR_WAIT(mbar_wait_warp, "mbarrier.try_wait.parity.shared::cta.b64", DLR_AGREE("P1"), DLR_AGREE("P2"))
+DLR_MBAR_WAIT(mbar_wait_warp, "mbarrier.try_wait.parity.shared::cta.b64", DLR_AGREE)
 // ... acquiring at cluster scope, for arrivals and stores that come from other CTAs
-DLR_MBAR_WAIT(mbar_wait_warp_cluster, "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64", DLR_AGREE("P1"), DLR_AGREE("P2"))
+DLR_MBAR_WAIT(mbar_wait_warp_cluster, "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64", DLR_AGREE)
 // For a single lane.
-DLR_MBAR_WAIT(mbar_wait_lane, "mbarrier.try_wait.parity.shared::cta.b64", "", "")
+DLR_MBAR_WAIT(mbar_wait_lane, "mbarrier.try_wait.parity.shared::cta.b64", "")
 #undef DLR_AGREE
 #undef DLR_MBAR_WAIT
 

@@ -35,9 +35,9 @@
 // apart.  Two terms of a row are the two columns a lane holds of an accumulator, the third is in the lane beside it.  Error
 // against 64 bits, output rounding included: d = 1024, 64 rows 1.6574e-3, 6e-5 to 9e-5 of the values on the other side of a
 // tie, both as decode_cluster.cu (rounded operands: 1.7133e-3, 0.18); d = 2048, 28 rows 1.6673e-3 (1.7225e-3).  Time (us,
-// rounded operands / terms / decode_cluster.cu): d = 1024, 8 rows 110 / 117 / 294; d = 2048, 17 rows 150 / 166 / 394.
+// rounded operands / terms / decode_cluster.cu): d = 1024, 8 rows 109 / 114 / 294; d = 2048, 28 rows 150 / 168 / 406.
 //
-// Measured on a B200 against the best kernel before it (us): d = 1024 (clusters of 4), 1 / 8 / 264 rows: 110 / 117 / 124
+// Measured on a B200 against the best kernel before it (us): d = 1024 (clusters of 4), 1 / 8 / 264 rows: 103 / 114 / 124
 // against 281 / 295 / 751; d = 2048 (8), 4 / 64 / 333 rows: 150 / 162 / 380 against 333 / 767 / 886; d = 4096 (16), 1 / 16 /
 // 64 rows: 222 / 236 / 357 against 323 / 521 / 1092; d = 5120 (16), 12 / 64 / 112 rows: 648 / 735 / 870 against 828 / 2350 /
 // 5555.
