@@ -301,15 +301,14 @@ dlr_stream_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     err_layer = uq;
                 }
             }
-            if (err || *abort_flag) {
-                // copies requested before giving up still land in this CTA's shared memory: wait for them
-                for (long long m = nh - 1; m >= 0 && m >= nh - int(kNH); --m)
-                    mbar_wait(smem_u32(&bars->h_full[m % kNH]), uint32_t(m / kNH) & 1u, kDrainPolls);
-                for (long long m = nu - 1; m >= 0 && m >= nu - int(NU); --m)
-                    mbar_wait(smem_u32(&bars->u_full[m % NU]), uint32_t(m / NU) & 1u, kDrainPolls);
-                for (long long m = nv - 1; m >= 0 && m >= nv - int(NV); --m)
-                    mbar_wait(smem_u32(&bars->v_full[m % NV]), uint32_t(m / NV) & 1u, kDrainPolls);
-            }
+            // the copies asked for land in this CTA's shared memory: wait for the last of every stage (always: the other
+            // warps may give up after this one is done)
+            for (long long m = nh - 1; m >= 0 && m >= nh - int(kNH); --m)
+                mbar_wait(smem_u32(&bars->h_full[m % kNH]), uint32_t(m / kNH) & 1u, kDrainPolls);
+            for (long long m = nu - 1; m >= 0 && m >= nu - int(NU); --m)
+                mbar_wait(smem_u32(&bars->u_full[m % NU]), uint32_t(m / NU) & 1u, kDrainPolls);
+            for (long long m = nv - 1; m >= 0 && m >= nv - int(NV); --m)
+                mbar_wait(smem_u32(&bars->v_full[m % NV]), uint32_t(m / NV) & 1u, kDrainPolls);
         }
     } else if (warp == 1) {
         // =============================== U-MMA warp ================================

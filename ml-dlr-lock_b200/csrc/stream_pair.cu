@@ -288,10 +288,10 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
                 ++nh;
                 if (++hc == nch) { hc = 0; if (++hq == p.L) { hq = -1; ++ht; } }
             }
-            // copies requested before giving up still land in shared memory: wait for them
-            if (err || *abort_flag)
-                for (long long m = nh - 1; m >= 0 && m >= nh - kBufs; --m)
-                    mbar_wait(smem_u32(&bars->dh_full[m % kBufs]), uint32_t(m / kBufs) & 1u, kDrainPolls);
+            // the copies asked for land in this CTA's shared memory: wait for the last ones (always, as below: the other
+            // warps may give up after this one is done)
+            for (long long m = nh - 1; m >= 0 && m >= nh - kBufs; --m)
+                mbar_wait(smem_u32(&bars->dh_full[m % kBufs]), uint32_t(m / kBufs) & 1u, kDrainPolls);
         }
     } else if (warp == kWarpU) {
         // =============================== TMA producer: U' ==========================
@@ -327,7 +327,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
             }
             // (the weight copies of both CTAs are counted in the leader, which the second CTA outlasts through the cluster
             // barrier)
-            if ((err || *abort_flag) && hf == 0)
+            if (hf == 0)
                 for (long long m = nu - 1; m >= 0 && m >= nu - int(NU); --m)
                     mbar_wait_cluster(smem_u32(&bars->u_full[m % NU]), uint32_t(m / NU) & 1u, kDrainPolls);
         }
@@ -361,7 +361,7 @@ dlr_stream_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
             }
             // (the weight copies of both CTAs are counted in the leader, which the second CTA outlasts through the cluster
             // barrier)
-            if ((err || *abort_flag) && hf == 0)
+            if (hf == 0)
                 for (long long m = nv - 1; m >= 0 && m >= nv - int(NV); --m)
                     mbar_wait_cluster(smem_u32(&bars->v_full[m % NV]), uint32_t(m / NV) & 1u, kDrainPolls);
         }

@@ -57,3 +57,31 @@ def test_cluster_kernel(d, r, L, M, stripe, monkeypatch):
 def test_pair_kernel(d, r, L, M, monkeypatch):
     monkeypatch.setenv("DLRB200_FORCE_PATH", "5")
     _check(d, r, L, M, 5)
+
+
+# the shortest waits on stacks that fit the rings whole: a call either says that it gave up or is right, and the next one works
+@pytest.mark.parametrize("path,d,r,L,M", [(2, 1024, 32, 1, 200), (4, 512, 64, 1, 65), (4, 512, 64, 2, 300), (4, 512, 256, 1, 129), (4, 1024, 128, 1, 200),
+                                          (5, 512, 64, 1, 600)])
+def test_a_call_that_gives_up_leaves_nothing_behind(path, d, r, L, M, monkeypatch):
+    import dlr_lock_b200 as D
+    monkeypatch.setenv("DLRB200_FORCE_PATH", str(path))
+    dev = torch.device("cuda:0")
+    p, x = O.seeded_case(d, r, L, M, seed=d + r + L, alpha=1.0, gain_jitter=0.1)
+    Vf, Uf = D.ops.fold_weights(p.V.to(dev), p.U.to(dev), p.w.to(dev), p.alpha.to(dev))
+    xd = x.to(dev)
+    want = D.ops.forward_folded(xd, Vf, Uf, p.eps)
+    torch.cuda.synchronize()
+    D.ops.check_status()
+    monkeypatch.setenv("DLRB200_SPIN_LIMIT", "1")
+    y = D.ops.forward_folded(xd, Vf, Uf, p.eps)
+    torch.cuda.synchronize()
+    monkeypatch.delenv("DLRB200_SPIN_LIMIT")
+    try:
+        D.ops.check_status()
+        assert torch.equal(y, want)
+    except D.ops._lib.DlrB200Error:
+        pass
+    y = D.ops.forward_folded(xd, Vf, Uf, p.eps)
+    torch.cuda.synchronize()
+    D.ops.check_status()
+    assert torch.equal(y, want)
