@@ -201,9 +201,7 @@ dlr_decode_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_
             // the stage leads a group; `lead` holds its next parity per stage, and the compute warps keep the same
             // bits.
             RingPos rp;
-            uint32_t lead = 0;
-            uint32_t last_bar[2] = {0, 0}, last_par[2] = {0, 0};   // the two youngest groups, for the drain below
-            bool any[2] = {false, false};
+            uint32_t lead = 0, led = 0;          // (led: stages that have led a group)
             for (l = 0; l < p.L && !err; ++l) {
                 uint32_t bar = 0;
                 for (int i = 0; i < kVT + C::UT; ++i, rp.step(uint32_t(S))) {
@@ -211,13 +209,10 @@ dlr_decode_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_
                     if (!wait_cta(smem_u32(&bars->empty[st]), rp.ph ^ 1u)) { err = DLRB200_ERR_TIMEOUT_COPY; break; }
                     const uint32_t dst = ring_s + st * kStage;
                     if (i == 0 || i == kVT) {
-                        const int grp = i == 0 ? 0 : 1;
                         bar = smem_u32(&bars->full[st]);
                         mbar_arrive_expect_tx(bar, i == 0 ? kVT * C::V_TILE_BYTES : C::UT * C::U_TILE_BYTES);
-                        last_bar[grp] = bar;
-                        last_par[grp] = (lead >> st) & 1u;
-                        any[grp] = true;
                         lead ^= 1u << st;
+                        led |= 1u << st;
                     }
                     if (i < kVT) {
                         tma_load_2d(dst, &tmV, stripe0 + 64 * i, l * R, bar);
@@ -232,11 +227,11 @@ dlr_decode_cluster_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_
                     *abort_flag = 1;
                     report_status(p.status, p.mirror, err | (l << 8));
                 }
-                // tiles already requested still land in this CTA's ring: wait (bounded) before leaving.  A group
-                // cut short by the error never completes its byte count; older groups have been consumed.
-                for (int g = 0; g < 2; ++g)
-                    if (any[g]) mbar_wait(last_bar[g], last_par[g], kDrainPolls);
             }
+            // the tiles asked for land in this CTA's ring: wait (bounded) for the last group of every stage before leaving,
+            // whatever the others do, who may give up after this.  A group cut short by an error never completes.
+            for (int st = 0; st < S; ++st)
+                if ((led >> st) & 1u) mbar_wait(smem_u32(&bars->full[st]), ((lead >> st) & 1u) ^ 1u, kDrainPolls);
         }
     } else {
         // =============================== compute warps ==============================

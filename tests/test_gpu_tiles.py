@@ -60,7 +60,7 @@ def test_pair_kernel(d, r, L, M, monkeypatch):
 
 
 # the shortest waits on stacks that fit the rings whole: a call either says that it gave up or is right, and the next one works
-@pytest.mark.parametrize("path,d,r,L,M", [(2, 1024, 32, 1, 200), (4, 512, 64, 1, 65), (4, 512, 64, 2, 300), (4, 512, 256, 1, 129), (4, 1024, 128, 1, 200),
+@pytest.mark.parametrize("path,d,r,L,M", [(2, 1024, 32, 1, 200), (3, 1024, 64, 1, 5), (3, 512, 32, 2, 64), (4, 512, 64, 1, 65), (4, 512, 64, 2, 300), (4, 512, 256, 1, 129), (4, 1024, 128, 1, 200),
                                           (5, 512, 64, 1, 600)])
 def test_a_call_that_gives_up_leaves_nothing_behind(path, d, r, L, M, monkeypatch):
     import dlr_lock_b200 as D
