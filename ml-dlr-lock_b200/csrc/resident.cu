@@ -35,10 +35,11 @@
 // apart.  Two terms of a row are the two columns a lane holds of an accumulator, the third is in the lane beside it.  Error
 // against 64 bits, output rounding included: d = 1024, 64 rows 1.6574e-3, 6e-5 to 9e-5 of the values on the other side of a
 // tie, both as decode_cluster.cu (rounded operands: 1.7133e-3, 0.18); d = 2048, 28 rows 1.6673e-3 (1.7225e-3).  Time (us,
-// rounded operands / terms / decode_cluster.cu): d = 1024, 8 rows 109 / 114 / 294; d = 2048, 28 rows 150 / 168 / 406.
+// terms / decode_cluster.cu): d = 1024, 8 rows 110 / 294; d = 2048, 28 rows 165 / 406 (a call of the other form with as many
+// rows: 6 % and 12 % less).
 //
-// Measured on a B200 against the best kernel before it (us): d = 1024 (clusters of 4), 1 / 8 / 264 rows: 103 / 114 / 124
-// against 281 / 295 / 751; d = 2048 (8), 4 / 64 / 333 rows: 150 / 162 / 380 against 333 / 767 / 886; d = 4096 (16), 1 / 16 /
+// Measured on a B200 against the best kernel before it (us): d = 1024 (clusters of 4), 1 / 8 / 264 rows: 100 / 110 / 124
+// against 281 / 295 / 751; d = 2048 (8), 4 / 64 / 333 rows: 140 / 162 / 390 against 333 / 767 / 886; d = 4096 (16), 1 / 16 /
 // 64 rows: 222 / 236 / 357 against 323 / 521 / 1092; d = 5120 (16), 12 / 64 / 112 rows: 648 / 735 / 870 against 828 / 2350 /
 // 5555.
 //
@@ -117,7 +118,7 @@ struct RBars {
     uint64_t rbar[2];          // partial z and sums of squares have arrived (bytes); BC: by parity of the layer
     uint64_t sbar;             // RS: s has arrived (bytes)
     int fail[2];               // by parity of the layer: a warp gave up before this layer's block barrier
-    int abort_flag, give_up;
+    int abort_flag;
 };
 static_assert(sizeof(RBars) <= 1024, "barrier block");
 
@@ -187,7 +188,6 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
         mbar_init(smem_u32(&bars->sbar), 1);
         fail[0] = fail[1] = 0;
         *abort_flag = 0;
-        bars->give_up = 0;
         fence_mbar_init();
         tma_prefetch_desc(&tmV);
         tma_prefetch_desc(&tmU);
@@ -435,8 +435,6 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             for (l = 0; l < p.L && !err; ++l) {
                 for (int s = 0; s < C::NVS; ++s) ask_v();
                 for (int s = 0; s < C::NUS; ++s) ask_u();
-                // the status word was set before this launch: give up
-                if (l == 0 && *reinterpret_cast<volatile int*>(p.status) != 0) *reinterpret_cast<volatile int*>(&bars->give_up) = 1;
             }
             // (whatever the others do: they may give up after this, with copies still on their way)
             drain_copies();
@@ -446,6 +444,8 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
         // columns stripe0 + 16 u + g (+8), rows 8 nt + 2t, + 1 of this cluster's rows; TERMS: h[i][0][0] only, columns
         // stripe0 + 16 u + 8 (t % 2) + g of row t / 2
         float h[C::UM][NT][4];
+        // (read with the input, which takes as long)
+        const int failed_before = *reinterpret_cast<volatile int*>(p.status);
         const int row_t = t >> 1, col_t = stripe0 + 32 * warp + 8 * (t & 1) + g;
         if constexpr (TERMS) {
 #pragma unroll
@@ -531,6 +531,9 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
 #pragma unroll
         for (int k = 0; k < PER; ++k) to_peer[k] = mapa(sb_s, uint32_t(k * NPART + part)) - sb_s;
         publish();
+        // the status word was set before this launch (or by another cluster of it): give up before the first layer, whose block
+        // barrier tells the whole CTA
+        if (__any_sync(0xffffffffu, failed_before != 0)) err = DLRB200_ERR_TIMEOUT_BARRIER;
 
 #pragma unroll 1
         for (l = 0; l < p.L; ++l) {
@@ -558,7 +561,6 @@ dlr_resident_kernel(const __grid_constant__ CUtensorMap tmV, const __grid_consta
             if (warp == NU - 1 && lane == 0) {
                 mbar_arrive_expect_tx(rbar_s, z_bytes + uint32_t(CS * 4 * rows));
                 if (!BC) mbar_arrive_expect_tx(sbar_s, uint32_t(rows * R * 2) * (TERMS ? 3u : 1u));
-                if (*reinterpret_cast<volatile int*>(&bars->give_up)) err = DLRB200_ERR_TIMEOUT_BARRIER;
             }
             __syncwarp();
             // ---- this layer's U' fragments, while the V warps work and the partials travel

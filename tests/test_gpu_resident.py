@@ -66,7 +66,7 @@ def test_pair_of_rows_in_fp32(d, r, L, M):
 
 # every kernel of every shape, on stacks that may be asked for whole before anyone gives up: copies still land while the rest
 # leaves
-@pytest.mark.parametrize("L", [6])
+@pytest.mark.parametrize("L", [1, 2, 6])
 @pytest.mark.parametrize("d,r,M", [(1024, 32, 1), (1024, 32, 8), (1024, 32, 267), (1024, 32, 530), (1024, 32, 1100), (2048, 64, 4), (2048, 64, 20),
                                    (2048, 64, 200), (2048, 64, 400), (4096, 128, 1), (4096, 128, 115), (4096, 128, 200), (5120, 256, 3),
                                    (5120, 256, 115), (5120, 256, 200)])
