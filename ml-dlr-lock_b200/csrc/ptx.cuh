@@ -184,10 +184,12 @@ struct RingPos {
     }
 };
 
-// A wait has given up: the first report stays in the status word, and goes to the host's copy of it if there is one.
+// A wait has given up: the first report stays in the status word, and every one puts it into the host's copy if there is one
+// (the host may have read and cleared that for an earlier launch, while the device word was still set for this one).
 __device__ __forceinline__ void report_status(int* status, int* mirror, int word) {
-    if (atomicCAS(status, 0, word) == 0 && mirror != nullptr) {
-        *reinterpret_cast<volatile int*>(mirror) = word;
+    const int first = atomicCAS(status, 0, word);
+    if (mirror != nullptr) {
+        *reinterpret_cast<volatile int*>(mirror) = first ? first : word;
         __threadfence_system();
     }
 }

@@ -92,8 +92,9 @@ def test_resident_kernel_gives_up_while_the_status_word_is_set(d, r, L, M, monke
     assert lib.dlrb200_forward(vp(xd), vp(out), vp(Vf), vp(Uf), M, d, r, L, 1e-6, vp(ent.ws), ent.ws.numel(), vp(ent.status), st) == 0
     torch.cuda.synchronize()
     assert bool((out == 7.0).all())
-    with pytest.raises(D.ops._lib.DlrB200Error):
-        D.ops.check_status()
+    with pytest.raises(D.ops._lib.DlrB200Error):                    # reported for this call too
+        D.ops.forward_folded(xd, Vf, Uf)
+    D.ops.check_status()                                            # and cleared
     y = D.ops.forward_folded(xd, Vf, Uf)
     torch.cuda.synchronize()
     D.ops.check_status()
