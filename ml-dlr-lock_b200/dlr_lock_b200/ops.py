@@ -37,6 +37,7 @@ class _Scratch:
         self.mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.word = ctypes.c_int.from_address(self.mirror.data_ptr())
         _lib.check(_lib.load().dlrb200_set_status_mirror(self.status_ptr, self.mirror.data_ptr()), "dlrb200_set_status_mirror")
+        _words.append((self.status, self.mirror))
         # workspaces that were outgrown: a CUDA graph captured earlier has their address in its nodes, so
         # they stay allocated for the life of the process (they are small: at most a few tens of MB)
         self.retired = []
@@ -52,6 +53,9 @@ class _Scratch:
 
 
 _workspaces: Dict[Tuple[int, int], _Scratch] = {}
+# status words and their mirrors, kept for the life of the process: the library knows the pair by address, and a CUDA graph
+# captured earlier has both in its nodes
+_words: list = []
 _derived: Dict[Tuple, Tuple[torch.Tensor, ...]] = {}
 _MIN_WORKSPACE = 1 << 20
 # the current stream of a device as an address, without building a stream object

@@ -549,6 +549,19 @@ def test_a_captured_graph_survives_a_later_larger_workspace(D):
     assert O.rel_l2(big.cpu(), O.forward_fp32(x[8:], p)) <= 1e-2
 
 
+def test_a_status_word_is_never_given_back(D):
+    # the library, and graphs captured earlier, go on writing to it and to its mirror
+    dev = torch.device("cuda:0")
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        net = D.PackedNet(torch.zeros(2, 32, 1024, device=dev, dtype=torch.bfloat16), torch.zeros(2, 1024, 32, device=dev, dtype=torch.bfloat16))
+        net(torch.zeros(1, 1024, device=dev, dtype=torch.bfloat16))
+        s.synchronize()
+        word = D.ops._workspaces.pop((0, s.cuda_stream)).status_ptr
+        later = [torch.zeros(1, dtype=torch.int32, device=dev) for _ in range(4096)]
+    assert word not in {t.data_ptr() for t in later}
+
+
 def test_a_device_timeout_surfaces_through_the_module_without_check_status(D, monkeypatch):
     # no explicit check_status: the forward mirrors the status word to pinned host memory on its stream and the
     # next forward on that stream raises
