@@ -3,8 +3,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <shared_mutex>
-#include <vector>
+#include <unordered_map>
 
 #include "cluster.h"
 #include "decode.h"
@@ -412,16 +413,14 @@ bool use_striped_clusters(int M, int d, int r, int L, const DevInfo& di) {
 
 namespace dlr {
 
-// (status word, host copy) pairs: one per stream a process uses
-struct Mirror { const int* status; int* host; };
-static std::vector<Mirror> g_mirrors;
+// status word -> host copy: one per stream a process uses, looked up at every launch
+static std::unordered_map<const int*, int*> g_mirrors;
 static std::shared_mutex g_mirrors_mutex;
 
 int* status_mirror(const int* status_dev) {
     std::shared_lock<std::shared_mutex> lock(g_mirrors_mutex);
-    for (const Mirror& m : g_mirrors)
-        if (m.status == status_dev) return m.host;
-    return nullptr;
+    const auto at = g_mirrors.find(status_dev);
+    return at == g_mirrors.end() ? nullptr : at->second;
 }
 
 bool encode_2d_bf16(void* encode_fn_ptr, CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
@@ -617,14 +616,13 @@ int dlrb200_status_to_host(const int* status_dev, int* status_host, void* stream
 int dlrb200_set_status_mirror(const int* status_dev, int* status_host) {
     if (!status_dev) return DLRB200_ERR_INVALID_ARG;
     std::unique_lock<std::shared_mutex> lock(dlr::g_mirrors_mutex);
-    auto& all = dlr::g_mirrors;
-    for (size_t i = 0; i < all.size(); ++i)
-        if (all[i].status == status_dev) {
-            if (status_host) all[i].host = status_host;
-            else all.erase(all.begin() + i);
-            return DLRB200_OK;
-        }
-    if (status_host) all.push_back({status_dev, status_host});
+    try {
+        if (status_host) dlr::g_mirrors[status_dev] = status_host;
+        else dlr::g_mirrors.erase(status_dev);
+    } catch (const std::bad_alloc&) {
+        g_last_cuda_error = int(cudaErrorMemoryAllocation);
+        return DLRB200_ERR_CUDA;
+    }
     return DLRB200_OK;
 }
 
