@@ -630,15 +630,22 @@ int dlrb200_fold_weights(const void* V, const void* U, const void* gain, const f
                          void* Up, int d, int r, int L, void* stream) {
     if (!V || !U || !gain || !alpha || !Vp || !Up || d <= 0 || r <= 0 || L <= 0) return DLRB200_ERR_INVALID_ARG;
     const size_t n = size_t(r) * d;
-    std::vector<const void*> at(size_t(4) * L);
-    for (int l = 0; l < L; ++l) {
-        at[l] = static_cast<const __nv_bfloat16*>(V) + l * n;
-        at[L + l] = static_cast<const __nv_bfloat16*>(U) + l * n;
-        at[2 * L + l] = static_cast<const __nv_bfloat16*>(gain) + size_t(l) * d;
-        at[3 * L + l] = alpha + l;
+    constexpr int kPart = 128;                  // layers at a time
+    const void* at[4][kPart];
+    for (int l0 = 0; l0 < L; l0 += kPart) {
+        const int layers = L - l0 < kPart ? L - l0 : kPart;
+        for (int i = 0; i < layers; ++i) {
+            const size_t l = size_t(l0 + i);
+            at[0][i] = static_cast<const __nv_bfloat16*>(V) + l * n;
+            at[1][i] = static_cast<const __nv_bfloat16*>(U) + l * n;
+            at[2][i] = static_cast<const __nv_bfloat16*>(gain) + l * d;
+            at[3][i] = alpha + l;
+        }
+        const int rc = dlrb200_fold_layers(at[0], at[1], at[2], at[3], DLRB200_FOLD_ALPHA_F32, static_cast<__nv_bfloat16*>(Vp) + l0 * n,
+                                           static_cast<__nv_bfloat16*>(Up) + l0 * n, d, r, layers, stream);
+        if (rc != DLRB200_OK) return rc;
     }
-    return dlrb200_fold_layers(at.data(), at.data() + L, at.data() + 2 * L, at.data() + 3 * L, DLRB200_FOLD_ALPHA_F32, Vp, Up, d, r, L,
-                               stream);
+    return DLRB200_OK;
 }
 
 int dlrb200_fold_layers(const void* const* V, const void* const* U, const void* const* gain, const void* const* alpha,
