@@ -542,7 +542,7 @@ struct CLaunch {
     // Clusters that can be resident at once on the current device (asked for once per device: the query and the opt-in to
     // large shared memory take longer than a launch), or -1.
     int max_clusters(int num_sms) const {
-        static std::atomic<int> known[kMaxDevices];          // 0: not asked yet
+        static std::atomic<int> known[kMaxDevices];          // 0: not known yet
         int dev = 0;
         if (stages < 2 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
         int n = known[dev].load(std::memory_order_acquire);
@@ -554,7 +554,7 @@ struct CLaunch {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
             (void)cudaGetLastError();
-            n = -1;
+            return -1;                                       // (not kept: it may have failed for a passing reason)
         }
         known[dev].store(n, std::memory_order_release);
         return n;

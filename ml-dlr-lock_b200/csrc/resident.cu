@@ -841,7 +841,7 @@ struct RLaunch {
     // Clusters that can be resident at once on the current device (asked for once per device: the query and the opt-in to
     // large shared memory take longer than a launch), or -1.
     int max_clusters() const {
-        static std::atomic<int> known[kMaxDevices];          // 0: not asked yet
+        static std::atomic<int> known[kMaxDevices];          // 0: not known yet
         int dev = 0;
         if (!smem || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
         int n = known[dev].load(std::memory_order_acquire);
@@ -854,7 +854,7 @@ struct RLaunch {
             (CS > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
             cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
             (void)cudaGetLastError();
-            n = -1;
+            return -1;                                       // (not kept: it may have failed for a passing reason)
         }
         known[dev].store(n, std::memory_order_release);
         return n;
