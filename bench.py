@@ -431,7 +431,7 @@ def sharded_block(dev, world, rank, barrier, Vp, Up, d, r, L, steps):
         t_local = time_steps(lambda: ops.forward_folded(xl, Vp, Up), n, 3, barrier) / n
         t_gather = time_steps(lambda: fwd.gather(ops.forward_folded(xl, Vp, Up), M), n, 3, barrier) / n
         t_full, t_local, t_gather = _max_over_ranks([t_full, t_local, t_gather], dev, world)
-        plan = ops.query_call(max(b - a, 1), d, r, L)
+        plan = ops.query(max(b - a, 1), d, r, L)
         out.append({"M": M, "rows_per_gpu": b - a, "ms_single_gpu_whole_batch": t_full, "ms_sharded_forward": t_local,
                     "ms_sharded_forward_and_gather": t_gather, "tokens_per_s_no_gather": M / (t_local * 1e-3),
                     "tokens_per_s_with_gather": M / (t_gather * 1e-3),
@@ -457,7 +457,7 @@ def decode_sweep(dev, name, Ms, peaks):
     rows = []
     for m in Ms:
         xm, ym = x[:m].contiguous(), torch.empty(m, d, device=dev, dtype=torch.bfloat16)
-        plan = ops.query_call(m, d, r, L)
+        plan = ops.query(m, d, r, L)
         if m <= 64:
             lo, med = min_latency_us(lambda: ops.forward_folded(xm, Vp, Up, out=ym))
             gbs = (wbytes + 4.0 * m * d) / (lo * 1e-6) / 1e9
@@ -591,7 +591,7 @@ def main():
     g.manual_seed(1000 + seed + rank)
     xs = [torch.randn(M, d, device=dev, generator=g).to(torch.bfloat16) for _ in range(2)]
     ys = [torch.empty_like(x) for x in xs]
-    plan = ops.query_call(M, d, r, L)
+    plan = ops.query(M, d, r, L)
     it = [0]
 
     def step():
@@ -755,7 +755,7 @@ def main():
             xm, ym = xs[0][:m].contiguous(), torch.empty(m, d, device=dev, dtype=torch.bfloat16)
             lo, med = min_latency_us(lambda: ops.forward_folded(xm, Vp, Up, out=ym))
             gbs = (wbytes + 4.0 * m * d) / (lo * 1e-6) / 1e9
-            dec.append({"M": m, "path": ops.query_call(m, d, r, L).path, "min_us": lo, "median_us": med, "us_per_layer": lo / L,
+            dec.append({"M": m, "path": ops.query(m, d, r, L).path, "min_us": lo, "median_us": med, "us_per_layer": lo / L,
                         "algorithmic_GBps": gbs, "frac_of_measured_hbm": gbs / peaks["hbm_gbs"], "tokens_per_s": m / (lo * 1e-6)})
         line["decode"] = dec
         pre = []
@@ -768,7 +768,7 @@ def main():
                 xm = torch.cat([xs[0]] * ((m + M - 1) // M))[:m].contiguous()
             ym = torch.empty(m, d, device=dev, dtype=torch.bfloat16)
             lo, med = min_latency_us(lambda: ops.forward_folded(xm, Vp, Up, out=ym), iters=10, warmup=3)
-            pl = ops.query_call(m, d, r, L)
+            pl = ops.query(m, d, r, L)
             pre.append({"M": m, "path": pl.path, "grid": pl.grid, "cluster": pl.cluster, "rounds": pl.passes, "min_us": lo,
                         "tokens_per_s": m / (lo * 1e-6), "TFLOPs": 4.0 * L * m * d * r / (lo * 1e-6) / 1e12})
             del xm, ym

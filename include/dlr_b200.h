@@ -98,16 +98,12 @@ DLRB200_API int dlrb200_last_cuda_error(void);
  * must not overlap on the GPU.  Returns 0 for an unsupported shape. */
 DLRB200_API size_t dlrb200_workspace_bytes(int M, int d, int r, int L);
 
-/* How the kernels that take any shape (paths 1 to 6) would run a forward of
- * this shape on the current device (the cluster kernel, path 2, with its stripe
- * of 512 columns).  Launches nothing.  Returns DLRB200_ERR_UNSUPPORTED_SHAPE /
- * _OCCUPANCY when they cannot. */
+/* How dlrb200_forward would run a call of this shape on the current device (and
+ * under the environment switches in force).  Launches nothing.  Returns
+ * DLRB200_ERR_UNSUPPORTED_SHAPE / _OCCUPANCY when it cannot. */
 DLRB200_API int dlrb200_query(int M, int d, int r, int L, dlrb200_plan* plan);
 
-/* What dlrb200_forward launches for a call of this shape: the plan of
- * dlrb200_query, or that of the resident-cluster kernel (path 7), which takes
- * small and medium batches of the shapes it is built for, or that of the cluster
- * kernel on twice the CTAs with a stripe of 256 columns. */
+/* The same under an earlier name. */
 DLRB200_API int dlrb200_query_call(int M, int d, int r, int L, dlrb200_plan* plan);
 
 /* y = DLRNet(x).

@@ -282,7 +282,7 @@ int large_batch_path(int M, int d, int r, int L, const DevInfo& di, double* esti
     if (can_cluster) {
         std::memset(&pl, 0, sizeof(pl));
         double us = 0.0;
-        if (dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, &pl, &us, false) == DLRB200_OK) {
+        if (dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, &pl, &us) == DLRB200_OK) {
             best = 0.97 * us;                            // ties go to the cluster kernel
             path = DLRB200_PATH_CLUSTER;
         }
@@ -486,6 +486,15 @@ int dlrb200_query(int M, int d, int r, int L, dlrb200_plan* plan) {
     if (rc != DLRB200_OK) return rc;
     std::memset(plan, 0, sizeof(*plan));
     plan->workspace_bytes = dlrb200_workspace_bytes(M, d, r, L);
+    // (in the order of dlrb200_forward)
+    if (M > 0) {
+        dlrb200_plan resident = *plan;
+        bool terms = false;
+        if (use_resident(M, d, r, L, di, &terms, &resident)) {
+            *plan = resident;
+            return DLRB200_OK;
+        }
+    }
     if (use_pair_path(M, d, r, L, di)) return dlr::stream_pair_plan(M, d, r, L, di.num_sms, di.smem_optin, plan);
     if (use_stream_path(M, d, r, L, di)) return dlr::stream_plan(M, d, r, L, di.num_sms, di.smem_optin, plan);
     if (use_striped_clusters(M, d, r, L, di)) {
@@ -494,7 +503,7 @@ int dlrb200_query(int M, int d, int r, int L, dlrb200_plan* plan) {
         plan->workspace_bytes = ws;
         return rc;
     }
-    if (use_cluster_path(M, d, r, L)) return dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, plan, nullptr, true);
+    if (use_cluster_path(M, d, r, L)) return dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, plan, nullptr);
     if (use_cluster_small(M, d, r)) return dlr::decode_cluster_plan(M, d, r, L, di.smem_optin, plan);
     const int dc = pick_stripe_cols(d, di.num_sms);
     if (dc == 0) return DLRB200_ERR_UNSUPPORTED_SHAPE;
@@ -507,17 +516,7 @@ int dlrb200_query(int M, int d, int r, int L, dlrb200_plan* plan) {
     return DLRB200_OK;
 }
 
-int dlrb200_query_call(int M, int d, int r, int L, dlrb200_plan* plan) {
-    const int rc = dlrb200_query(M, d, r, L, plan);
-    if (rc != DLRB200_OK || M == 0) return rc;
-    DevInfo di;
-    if (device_info(&di) != DLRB200_OK) return DLRB200_ERR_CUDA;
-    dlrb200_plan resident = *plan;
-    bool terms = false;
-    if (use_resident(M, d, r, L, di, &terms, &resident)) *plan = resident;
-    else if (plan->path == DLRB200_PATH_CLUSTER) return dlr::cluster_plan(M, d, r, L, di.num_sms, di.smem_optin, plan, nullptr, false);
-    return DLRB200_OK;
-}
+int dlrb200_query_call(int M, int d, int r, int L, dlrb200_plan* plan) { return dlrb200_query(M, d, r, L, plan); }
 
 int dlrb200_forward(const void* x, void* y, const void* Vp, const void* Up, int M, int d, int r, int L,
                     float eps, void* workspace, size_t workspace_bytes, int* status_dev, void* stream) {

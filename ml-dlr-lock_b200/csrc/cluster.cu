@@ -614,7 +614,7 @@ constexpr double layer_us(int r, int w) {
 // first that need two waves of clusters of 4) 567 / 885; d = 2048, r = 64: 1000 rows 734 / 554, 2000 rows 735 / 1096.
 // DLRB200_CLUSTER_STRIPE=256 or 512 overrides the choice.
 template <int R, int CS>
-int pick_stripe(const CArgs& a, dlrb200_plan* plan_only, double* us, bool wide_only) {
+int pick_stripe(const CArgs& a, dlrb200_plan* plan_only, double* us) {
     const CLaunch<R, CS, 512> wide(a.smem_optin);
     const int ww = wide.waves(a.M, a.num_sms);
     const double tw = ww ? ww * layer_us(R, 512) * a.L : 1e30;
@@ -626,8 +626,7 @@ int pick_stripe(const CArgs& a, dlrb200_plan* plan_only, double* us, bool wide_o
         if (const char* e = std::getenv("DLRB200_CLUSTER_STRIPE")) forced = std::atoi(e);
         if (forced ? (forced == 256 && wn) : tn < tw) {
             if (us) *us = tn;
-            if (!wide_only) return narrow.run(a, plan_only);
-            return wide.run(a, plan_only);
+            return narrow.run(a, plan_only);
         }
     }
     if (us) *us = tw;
@@ -641,9 +640,9 @@ bool combo_ok(int r, int cs) {
     return r >= 16 * cs;
 }
 
-int dispatch(const CArgs& a, int r, dlrb200_plan* plan_only, double* us, bool wide_only) {
+int dispatch(const CArgs& a, int r, dlrb200_plan* plan_only, double* us) {
 #define DLR_CASE(RR, CC) \
-    if (r == RR && a.d == CC * 512) return pick_stripe<RR, CC>(a, plan_only, us, wide_only);
+    if (r == RR && a.d == CC * 512) return pick_stripe<RR, CC>(a, plan_only, us);
     DLR_CASE(32, 1)
     DLR_CASE(32, 2)
     DLR_CASE(64, 1)
@@ -675,11 +674,11 @@ bool cluster_supported(int d, int r, int L) {
 
 size_t cluster_workspace_bytes(int, int, int, int) { return profiling() ? kProfBytes : 0; }
 
-int cluster_plan(int M, int d, int r, int L, int num_sms, int smem_optin, dlrb200_plan* plan, double* us, bool wide) {
+int cluster_plan(int M, int d, int r, int L, int num_sms, int smem_optin, dlrb200_plan* plan, double* us) {
     const size_t ws = plan->workspace_bytes;
     CArgs a{};
     a.M = M; a.d = d; a.L = L; a.num_sms = num_sms; a.smem_optin = smem_optin;
-    const int rc = dispatch(a, r, plan, us, wide);
+    const int rc = dispatch(a, r, plan, us);
     plan->workspace_bytes = ws;
     return rc;
 }
@@ -693,7 +692,7 @@ int cluster_forward(void* encode_fn_ptr, const void* x, void* y, const void* Vp,
         prof = reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(workspace) + 256);
     }
     const CArgs a{encode_fn_ptr, x, y, Vp, Up, M, d, L, eps, status_dev, stream, num_sms, smem_optin, spin_limit, prof};
-    return dispatch(a, r, nullptr, nullptr, false);
+    return dispatch(a, r, nullptr, nullptr);
 }
 
 }  // namespace dlr

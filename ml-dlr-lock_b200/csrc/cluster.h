@@ -20,8 +20,8 @@ int* status_mirror(const int* status_dev);
 
 bool cluster_supported(int d, int r, int L);
 size_t cluster_workspace_bytes(int M, int d, int r, int L);
-// `us`: estimated time, or null.  `wide`: the plan with a stripe of 512 columns, whichever a call takes.
-int cluster_plan(int M, int d, int r, int L, int num_sms, int smem_optin, dlrb200_plan* plan, double* us, bool wide);
+// `us`: estimated time, or null.
+int cluster_plan(int M, int d, int r, int L, int num_sms, int smem_optin, dlrb200_plan* plan, double* us);
 int cluster_forward(void* encode_fn_ptr, const void* x, void* y, const void* Vp, const void* Up, int M, int d,
                     int r, int L, float eps, void* workspace, int* status_dev, cudaStream_t stream, int num_sms,
                     int smem_optin, unsigned int spin_limit);

@@ -821,7 +821,7 @@ int launch_pair(void* enc, const void* x, void* y, const void* Vp, const void* U
         plan_only->path = DLRB200_PATH_STREAMED_PAIRS;
         plan_only->grid = grid;
         plan_only->cluster = 2 * pp;
-        plan_only->stripe_cols = 128;
+        plan_only->stripe_cols = kCWP;
         plan_only->rows_per_pass = 2 * kRowsP;
         plan_only->passes = (num_tiles + clusters - 1) / clusters;
         plan_only->stages = C::NU + C::NV;

@@ -171,18 +171,13 @@ def forward_host(x_host: torch.Tensor, y_host: torch.Tensor, x_dev: torch.Tensor
 
 
 def query(M: int, d: int, r: int, L: int) -> _lib.Plan:
-    """How the kernels for any shape would run a forward of this shape on the current CUDA device (``query_call``: what
-    a call launches)."""
+    """What ``forward_folded`` launches for a call of this shape on the current CUDA device."""
     plan = _lib.Plan()
     _lib.check(_lib.load().dlrb200_query(M, d, r, L, ctypes.byref(plan)), "dlrb200_query")
     return plan
 
 
-def query_call(M: int, d: int, r: int, L: int) -> _lib.Plan:
-    """What ``forward_folded`` launches for a call of this shape on the current CUDA device."""
-    plan = _lib.Plan()
-    _lib.check(_lib.load().dlrb200_query_call(M, d, r, L, ctypes.byref(plan)), "dlrb200_query_call")
-    return plan
+query_call = query          # (an earlier name)
 
 
 def fold_weights(V: torch.Tensor, U: torch.Tensor, gain: torch.Tensor, alpha: torch.Tensor):

@@ -3,7 +3,7 @@
 ``B_hi``, ``kernel``, ``callable`` (importable dotted path), ``config`` and
 ``note``.  This build has one backend behind one callable; it covers every batch
 size of all four model shapes.  The library picks among its device paths per
-call (``dlrb200_query_call`` reports the choice for a shape on the current device);
+call (``dlrb200_query`` reports the choice for a shape on the current device);
 the ranges below name the path that serves most of each range on a B200, and
 ``describe`` fills an entry from the library's own answer.
 """
@@ -33,7 +33,7 @@ PATH_CONFIGS = {
 
 def _entry(lo, hi, path, note):
     return {"B_lo": lo, "B_hi": hi, "kernel": PATH_NAMES[path], "callable": _CALLABLE,
-            "config": PATH_CONFIGS[path] + "; picked per call by dlrb200_query_call", "note": note}
+            "config": PATH_CONFIGS[path] + "; picked per call by dlrb200_query", "note": note}
 
 
 def _entries(name):
@@ -71,7 +71,7 @@ def describe(model: str, batch_size: int, depth: int):
     if entry is None:
         return None
     cfg = MODEL_CONFIGS[model]
-    plan = ops.query_call(batch_size, cfg["d"], cfg["r"], depth)
+    plan = ops.query(batch_size, cfg["d"], cfg["r"], depth)
     out = dict(entry)
     out["kernel"] = PATH_NAMES.get(plan.path, f"path{plan.path}")
     out["config"] = (f"{PATH_CONFIGS.get(plan.path, '')}; grid {plan.grid}, cluster {plan.cluster}, "

@@ -30,25 +30,25 @@ CFG = {  # d, r, L, seed  (the four single-net benchmark configurations)
     "cfg4": (5120, 256, 149, 3),
 }
 
-STRIPED, CLUSTER, CLUSTER_SMALL, STREAMED, STREAMED_PAIRS = 1, 2, 3, 4, 5
+STRIPED, CLUSTER, STREAMED, STREAMED_PAIRS, RESIDENT = 1, 2, 4, 5, 7
 
 # (configuration, rows, expected path, expected cluster size or None, expected grid or None)
 CASES = [
-    ("cfg1", 2048, CLUSTER, 2, None),
-    ("cfg2", 1, STRIPED, 1, 32),
-    ("cfg2", 4, STRIPED, 1, 32),
-    ("cfg2", 16, STRIPED, 1, 32),
-    ("cfg2", 64, None, None, None),
-    ("cfg3", 1, STRIPED, 1, 64),
-    ("cfg3", 16, STRIPED, 1, 64),
-    ("cfg3", 64, None, None, None),
-    ("cfg3", 1024, None, None, None),
+    ("cfg1", 2048, CLUSTER, 4, 64),
+    ("cfg2", 1, RESIDENT, 8, 8),
+    ("cfg2", 4, RESIDENT, 8, 16),
+    ("cfg2", 16, RESIDENT, 8, 64),
+    ("cfg2", 64, RESIDENT, 8, None),
+    ("cfg3", 1, RESIDENT, 16, 16),
+    ("cfg3", 16, RESIDENT, 16, None),
+    ("cfg3", 64, RESIDENT, 16, None),
+    ("cfg3", 1024, CLUSTER, 8, 64),
     ("cfg3", 2048, STREAMED_PAIRS, 8, 64),
     ("cfg3", 4096, STREAMED, None, None),
     ("cfg3", 8192, STREAMED_PAIRS, 4, 128),
     ("cfg3", 16384, STREAMED_PAIRS, 4, None),
     ("cfg4", 1, STRIPED, 1, 80),
-    ("cfg4", 64, STRIPED, 1, 80),
+    ("cfg4", 64, RESIDENT, 16, None),
     ("cfg4", 4096, STREAMED, None, None),
 ]
 

@@ -183,7 +183,7 @@ def test_abi_argument_errors(D):
     assert lib.dlrb200_forward(*args(x=vp(y))) == 1             # aliasing
     torch.cuda.synchronize()
     plan = D.ops.query(4, 4096, 128, 143)
-    assert plan.path == 1 and plan.stripe_cols == 64 and plan.grid == 64
+    assert plan.path == 7 and plan.stripe_cols == 256 and plan.grid == 32        # two clusters of 16, two rows each
 
 
 def test_host_buffer_entry_point(D):
@@ -333,11 +333,17 @@ def test_streamed_path_is_chosen_where_it_is_faster_or_alone(D):
     assert q(16384, 2048, 64, 142).path == 5
     assert q(8192, 512, 64, 60).path == 2         # a cluster of one CTA has no exchange to lose time in
     assert q(4096, 5120, 256, 149).path == 4      # rank 256: one tensor-memory buffer, still streamed
-    assert q(16, 4096, 128, 143).path == 1        # counted exchange through L2
-    assert q(40, 4096, 128, 143).path == 6        # more rows: clusters of 8 reduce among themselves first
-    assert q(64, 4096, 128, 143).path == 6 and q(64, 4096, 128, 143).cluster == 8
-    assert q(64, 1024, 32, 141).path == 3 and q(20, 2048, 64, 142).path == 3 and q(40, 2048, 64, 142).path == 6
-    assert q(64, 5120, 256, 149).path == 1        # does not fit the two-level kernel's shared memory
+    # small and medium batches of the shapes the resident kernel is built for
+    for M, d, r, L in ((1, 1024, 32, 141), (64, 1024, 32, 141), (600, 1024, 32, 141), (20, 2048, 64, 142), (333, 2048, 64, 142),
+                       (1, 4096, 128, 143), (64, 4096, 128, 143), (12, 5120, 256, 149), (300, 5120, 256, 149)):
+        assert q(M, d, r, L).path == 7 and q(M, d, r, L).cluster == d // q(M, d, r, L).stripe_cols
+    # other small batches
+    assert q(4, 5120, 256, 149).path == 1         # 80 CTAs pull the weights faster than 16
+    assert q(16, 4096, 64, 143).path == 1         # counted exchange through L2
+    assert q(40, 4096, 64, 143).path == 6 and q(40, 4096, 64, 143).cluster == 8      # clusters of 8 reduce among themselves first
+    assert q(64, 1024, 64, 141).path == 3 and q(20, 2048, 128, 142).path == 3 and q(40, 2048, 128, 142).path == 6
+    assert q(40, 4096, 256, 20).path == 1         # does not fit the two-level kernel's shared memory
+    assert D.ops.query_call is D.ops.query
 
 
 def test_streamed_path_several_tiles_per_cta_and_identity(D, monkeypatch):

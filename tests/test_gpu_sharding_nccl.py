@@ -43,8 +43,9 @@ def _worker(rank, world, port, out_dir):
         ops.check_status()
         a, b = drv.local_rows(M)
         # the sharded result against the oracle always; against the single-GPU launch bit for bit when both run the
-        # same kernel (a block of another size may be routed to another kernel: same math, not the same bits)
-        same_path = ops.query(max(b - a, 1), d, r, L).path == ops.query(M, d, r, L).path
+        # same kernel in the same form (a block of another size may be routed to another one: same math, not the same bits)
+        form = lambda q: (q.path, q.cluster, q.stripe_cols, q.smem_bytes)
+        same_path = form(ops.query(max(b - a, 1), d, r, L)) == form(ops.query(M, d, r, L))
         ok[(d, M)] = dict(bits=bool(torch.equal(y, y_one)), same_path=same_path, rows=(a, b),
                           err=O.rel_l2(y.cpu(), O.forward_fp32(x, p)), shape=tuple(y.shape))
     torch.save(ok, os.path.join(out_dir, f"r{rank}.pt"))
