@@ -37,7 +37,7 @@ def _run(D, p, x):
                                   "cfg2_d2048_r64", "cfg3_d4096_r128", "cfg4_d5120_r256"])
 @pytest.mark.parametrize("path", ["default", "striped"])
 def test_small_batch_against_reference_fixtures(D, name, path, monkeypatch):
-    # default: the cluster small-batch kernel where the shape allows it; striped: forced
+    # default: the resident kernel or the cluster small-batch kernel where the shape allows it; striped: forced
     if path == "striped":
         monkeypatch.setenv("DLRB200_FORCE_PATH", "1")
     g = load_golden(name)
@@ -49,6 +49,19 @@ def test_small_batch_against_reference_fixtures(D, name, path, monkeypatch):
     Vo, Uo = O.fold_weights(p)
     assert torch.equal(Vf, Vo) and torch.equal(Uf, Uo)
     assert O.rel_l2(y, g["y_bf16"]) <= (TOL_TOTAL if m["alpha"] < 0.5 else 2.5e-2)
+    assert O.rel_l2(y, g["y_fp32"]) <= TOL_TOTAL
+    assert O.rel_l2_update_q(y, g["y_fp32"], x) <= TOL_UPDATE_FP32H
+
+
+@pytest.mark.parametrize("name", ["toy_d256_r32", "toy_d512_r64_stress", "cfg1_d1024_r32", "cfg1_d1024_r32_stress", "cfg2_d2048_r64"])
+def test_cluster_small_kernel_against_reference_fixtures(D, name, monkeypatch):
+    # (two of these shapes are the resident kernel's by default)
+    monkeypatch.setenv("DLRB200_FORCE_PATH", "3")
+    g = load_golden(name)
+    m = g["meta"]
+    assert D.ops.query(m["M"], m["d"], m["r"], m["L"]).path == 3
+    p, x = O.seeded_case(m["d"], m["r"], m["L"], m["M"], m["seed"], m["alpha"], m["gain_jitter"])
+    y, _, _ = _run(D, p, x)
     assert O.rel_l2(y, g["y_fp32"]) <= TOL_TOTAL
     assert O.rel_l2_update_q(y, g["y_fp32"], x) <= TOL_UPDATE_FP32H
 
