@@ -36,20 +36,23 @@ def _entry(lo, hi, path, note):
             "config": PATH_CONFIGS[path] + "; picked per call by dlrb200_query", "note": note}
 
 
+# (first batch size, path) per width, at the depth of the SwiGLU budget.  Bounds between two paths move by some rows with the
+# number of clusters that fit the GPU at once; from 4096 rows on, the large-batch kernels change places where a last wave of
+# tiles would be nearly empty.
+_RANGES = {1024: [(1, 7), (1057, 2)], 2048: [(1, 7), (481, 2), (5889, 5)], 4096: [(1, 7), (225, 2), (1921, 5), (3841, 4), (4225, 2), (5889, 5)],
+           5120: [(1, 1), (12, 7), (449, 4)]}
+_LAST = 131072
+_NOTES = {1: "A few rows of the widest model: all SMs pull the weights.",
+          2: "Row tiles on tensor cores, activations in tensor memory, one launch for all layers.",
+          4: "Row tiles on tensor cores, activations streamed, one launch for all layers.",
+          5: "256-row tiles on CTA pairs, activations streamed, one launch for all layers.",
+          7: "Small and medium batches: a few rows per cluster in registers, one launch for all layers."}
+
+
 def _entries(name):
-    d, r = MODEL_CONFIGS[name]["d"], MODEL_CONFIGS[name]["r"]
-    small = 3 if d <= 1024 else 1
-    big = 2 if r < 64 or d <= 2048 else 4
-    rows = [_entry(1, 64, small, "Small batch: one launch walks all layers, one exchange per layer.")]
-    if d >= 2048:
-        split = 17 if d >= 4096 else 29          # from where the two-level exchange is the faster one
-        rows = [_entry(1, split - 1, small, "Small batch: one launch walks all layers, one exchange per layer."),
-                _entry(split, 64, 6, "Small batch, more rows: the exchange in two levels.")]
-    big_pairs = 5 if r in (64, 128) else big
-    return rows + [
-        _entry(65, 4095, big, "Large batch: row tiles on tensor cores, one launch for all layers."),
-        _entry(4096, 131072, big_pairs, "Largest batches: 256-row tiles on CTA pairs where the shape allows."),
-    ]
+    ranges = _RANGES[MODEL_CONFIGS[name]["d"]]
+    ends = [lo - 1 for lo, _ in ranges[1:]] + [_LAST]
+    return [_entry(lo, hi, path, _NOTES[path]) for (lo, path), hi in zip(ranges, ends)]
 
 
 REGISTRY = {name: _entries(name) for name in MODEL_CONFIGS}
