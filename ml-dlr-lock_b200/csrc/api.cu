@@ -367,7 +367,7 @@ bool use_cluster_small(int M, int d, int r) {
 // The fewest rows of the striped kernel with the two-level exchange (below).
 int striped_clusters_from(int d, int r) { return d >= 4096 ? (r >= 256 ? 16 : 17) : (d >= 2048 ? 29 : 65); }
 
-// Calls that the resident-cluster kernel serves instead of the kernel planned above, where it covers the shape: batches of
+// Calls that the resident-cluster kernel serves instead of the others here, where it covers the shape: batches of
 // up to 64 rows (measured against the best of the others, us: d = 1024 100 / 281 at one row, 111 / 295 at 64; d = 2048
 // 151 / 332 at 8, 162 / 767 at 64; d = 4096 224 / 323 at one row, 237 / 524 at 16, 360 / 1093 at 64; at d = 5120 each of its
 // 16 CTAs pulls 328 KB a layer and the striped kernel's 80 are faster up to a dozen rows: 674 / 445 at one row, 648 / 828 at

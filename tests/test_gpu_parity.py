@@ -582,7 +582,7 @@ def test_a_status_word_is_never_given_back(D):
 
 
 def test_a_device_timeout_surfaces_through_the_module_without_check_status(D, monkeypatch):
-    # no explicit check_status: the forward mirrors the status word to pinned host memory on its stream and the
+    # no explicit check_status: the kernel that gives up writes the status word to pinned host memory as well, and the
     # next forward on that stream raises
     dev = torch.device("cuda:0")
     torch.manual_seed(3)
